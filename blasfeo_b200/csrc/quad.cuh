@@ -43,7 +43,7 @@ __device__ __forceinline__ void cpa_wait_all() { asm volatile("cp.async.wait_gro
 // pivot of column J < m goes to dA[J * IL] (HBM, when act) and, when PARK, to
 // ism[(32 / G) * J] (shared memory); bad = first J < m with a non-positive
 // pivot, plus one.  Columns >= m must hold an identity block (they factor to
-// it).
+// it).  Entries right of the diagonal come out undefined.
 template <int G>
 __device__ __forceinline__ int gowner(int lane, int i) { return (lane & ~(G - 1)) | (i & (G - 1)); }
 
@@ -53,26 +53,26 @@ struct GCol {
 	                                           bool act, int &bad) {
 		constexpr int R = 16 / G;
 		constexpr int SJ = J / G;
-		const double mine = (o == J % G) ? S[SJ][J] : 0.0;
-		const double c = __shfl_sync(0xffffffffu, mine, gowner<G>(lane, J));
+		const double c = __shfl_sync(0xffffffffu, S[SJ][J], gowner<G>(lane, J));
 		const bool ok = c > 0.0;
 		const double iv = ok ? rsqrt(c) : 0.0;
 		if (!ok && J < m && bad == 0) bad = J + 1;
+		// entries right of the diagonal are scaled and updated with the rest
+		// (nothing reads them): no predicate per entry
+#pragma unroll
+		for (int s = 0; s < R; s++)
+			if (J <= G * s + G - 1) S[s][J] *= iv;
 		if (o == J % G) {
-			S[SJ][J] = ok ? c * iv : 0.0;
+			if (!ok) S[SJ][J] = 0.0;
 			if (PARK) ism[(32 / G) * J] = iv;
 			if (act && J < m) dA[J * IL] = iv;
 		}
 #pragma unroll
-		for (int s = 0; s < R; s++)
-			if (J <= G * s + G - 1 && o + G * s > J) S[s][J] *= iv;
-#pragma unroll
 		for (int l = J + 1; l < 16; l++) {
-			const double own = (o == l % G) ? S[l / G][J] : 0.0;
-			const double llj = __shfl_sync(0xffffffffu, own, gowner<G>(lane, l));
+			const double llj = __shfl_sync(0xffffffffu, S[l / G][J], gowner<G>(lane, l));
 #pragma unroll
 			for (int s = 0; s < R; s++)
-				if (l <= G * s + G - 1 && o + G * s >= l) S[s][l] = fma(-S[s][J], llj, S[s][l]);
+				if (l <= G * s + G - 1) S[s][l] = fma(-S[s][J], llj, S[s][l]);
 		}
 		GCol<G, J + 1, PARK>::run(S, o, lane, m, ism, dA, act, bad);
 	}
@@ -85,30 +85,6 @@ struct GCol<G, 16, PARK> {
 // the quad form (G = 4) used by the n = 16 chain
 template <int J, bool PARK>
 using QCol = GCol<4, J, PARK>;
-
-// S[s][j] += sum over c < nc of W(o + G s, c) W(j, c) for a group of G lanes,
-// W column-major in shared memory: W(i, c) at w[16 c + i][t] (rows >= mrow
-// read as zero).  Column c is read by broadcast; the lane's own entries are
-// 16 consecutive slots over the group (no bank conflict).  Entries
-// j > o + G s are computed and left for the caller to clear.
-template <int G, int P>
-__device__ __forceinline__ void syrk_rows_cm(double (&S)[16 / G][16], const double (*w)[P], int nc, int mrow, int o,
-                                             int t) {
-	constexpr int R = 16 / G;
-#pragma unroll 2
-	for (int c = 0; c < nc; c++) {
-		double col[16], ai[R];
-#pragma unroll
-		for (int i = 0; i < 16; i++) col[i] = (i < mrow) ? w[16 * c + i][t] : 0.0;
-#pragma unroll
-		for (int s = 0; s < R; s++) ai[s] = (o + G * s < mrow) ? w[16 * c + o + G * s][t] : 0.0;
-#pragma unroll
-		for (int s = 0; s < R; s++)
-#pragma unroll
-			for (int j = 0; j < 16; j++)
-				if (j <= G * s + G - 1) S[s][j] = fma(ai[s], col[j], S[s][j]);
-	}
-}
 
 // clear the entries right of the diagonal of the group's rows, optionally
 // adding `shift` on the diagonal.  Selects, not conditional stores: a store
@@ -123,27 +99,6 @@ __device__ __forceinline__ void clear_upper_g(double (&S)[16 / G][16], int o, do
 			const double v = S[s][j] + ((j == o + G * s) ? shift : 0.0);
 			S[s][j] = (j > o + G * s) ? 0.0 : v;
 		}
-}
-
-// S[s][j] += sum over the columns c < nc of W(q + 4s, c) W(j, c), W read from
-// shared memory at w[16 i + c][t] (rows >= mrow read as zero): the syrk of the
-// quad's rows, entries j > q + 4s computed and left for the caller to clear
-__device__ __forceinline__ void syrk_rows(double (&S)[4][16], const double (*w)[QPW], int nc, int mrow, int q,
-                                          int t) {
-#pragma unroll 2
-	for (int c = 0; c < nc; c++) {
-		double col[16];
-#pragma unroll
-		for (int i = 0; i < 16; i++) col[i] = (i < mrow) ? w[16 * i + c][t] : 0.0;
-#pragma unroll
-		for (int s = 0; s < 4; s++) {
-			const double ai =
-			    (q == 0) ? col[4 * s] : (q == 1) ? col[4 * s + 1] : (q == 2) ? col[4 * s + 2] : col[4 * s + 3];
-#pragma unroll
-			for (int j = 0; j < 16; j++)
-				if (j <= 4 * s + 3) S[s][j] = fma(ai, col[j], S[s][j]);
-		}
-	}
 }
 
 // the quad form of clear_upper_g

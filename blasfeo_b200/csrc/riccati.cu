@@ -1,5 +1,7 @@
-// Batched Riccati recursion (LQR backward factorization), one warp per
-// problem, the whole recursion in one persistent kernel.
+// Batched Riccati recursion (LQR backward factorization) on back-to-back
+// slabs: FP64 by the tensor-core kernel of riccati_core.cuh, FP32 by the
+// kernel below, one warp per problem, the whole recursion in one persistent
+// kernel.
 //
 // Per problem (examples/example_d_riccati_recursion.c:115-143,
 // d_back_ric_trf_libstr):
@@ -14,15 +16,16 @@
 // the reference example does with nu_N = 0.
 //
 // The factor of stage k+1 never leaves the chip: it is kept in shared memory
-// (FP64) and consumed by stage k.  Each stage's BAbt_k and RSQ_k are bulk
+// and consumed by stage k.  Each stage's BAbt_k and RSQ_k are bulk
 // copied (TMA) into a double buffer so the next stage's inputs arrive while
 // the current stage computes; L_k (lower triangle) and its inverse diagonal
 // are the only writes.  nu + nx <= 16: lane i owns row i; the 16x16 factor
-// runs in FP64 registers (DiagCol, chol.cuh).  T = float gives the
-// single-precision variant (FP32 storage and FP32 trmm/syrk products; the
-// pivots and rank-1 updates of the diagonal factor stay FP64).
+// runs in FP64 registers (DiagCol, chol.cuh).  FP32 storage and FP32
+// trmm/syrk products; the pivots and rank-1 updates of the diagonal factor
+// stay FP64.
 #include "chol.cuh"
 #include "common.cuh"
+#include "riccati_core.cuh"
 #include "tma.cuh"
 
 namespace {
@@ -171,6 +174,46 @@ __global__ void __launch_bounds__(RIC_WARPS * 32) k_ric_trf(int batch, int N, in
 	}
 }
 
+// FP64: 4,096 problems, N = 30, nx = 12, nu = 4: a warp per problem as in
+// k_ric_trf 0.88 ms, k_ric_trf_dmma 0.23 ms
+int ric_launch(int batch, int N, int nx, int nu, struct blasfeo_dmat_batch *sBA, struct blasfeo_dmat_batch *sRSQ,
+               struct blasfeo_dmat_batch *sL, int *info, cudaStream_t s) {
+	ric::Args a;
+	a.batch = batch;
+	a.N = N;
+	a.nx = nx;
+	a.nu = nu;
+	a.cnx = (nx + 3) / 4 * 4;
+	a.BA = N > 0 ? sBA->pA : nullptr;
+	a.RSQ = sRSQ->pA;
+	a.L = sL->pA;
+	a.Ld = sL->dA;
+	a.sba = N > 0 ? sBA->stride : 0;
+	a.srsq = sRSQ->stride;
+	a.sl = sL->stride;
+	a.bs = 0;
+	a.info = info;
+	return ric::launch<false>(a, s);
+}
+
+int ric_launch(int batch, int N, int nx, int nu, struct blasfeo_smat_batch *sBA, struct blasfeo_smat_batch *sRSQ,
+               struct blasfeo_smat_batch *sL, int *info, cudaStream_t s) {
+	if (info) cudaMemsetAsync(info, 0, sizeof(int) * batch, s);
+	const RicLayout<float> lay = ric_layout<float>(nx);
+	const size_t smem = (size_t)lay.warp_bytes * RIC_WARPS;
+	cudaFuncSetAttribute(k_ric_trf<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	int per_sm = 0;
+	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ric_trf<float>, RIC_WARPS * 32, smem);
+	if (per_sm < 1) per_sm = 1;
+	long long grid = (long long)bf::num_sms() * per_sm;
+	const long long need = (batch + RIC_WARPS - 1) / RIC_WARPS;
+	if (grid > need) grid = need;
+	k_ric_trf<float><<<(unsigned)grid, RIC_WARPS * 32, smem, s>>>(
+	    batch, N, nx, nu, N > 0 ? sBA->pA : nullptr, N > 0 ? sBA->stride : 0, sRSQ->pA, sRSQ->stride, sL->pA, sL->dA,
+	    sL->stride, info, bf::wait_limit());
+	return bf::check_launch();
+}
+
 template <typename T, typename BT>
 int ric_run(int batch, int N, int nx, int nu, BT *sBA, BT *sRSQ, BT *sL, int *info, void *stream) {
 	if (batch < 0 || N < 0 || nx < 1 || nu < 0 || !sRSQ || !sL || (N > 0 && !sBA)) return BLASFEO_B200_EINVAL;
@@ -184,21 +227,8 @@ int ric_run(int batch, int N, int nx, int nu, BT *sBA, BT *sRSQ, BT *sL, int *in
 		return BLASFEO_B200_EINVAL;
 	if (((uintptr_t)sRSQ->pA & 15) || ((sRSQ->stride * sizeof(T)) & 15)) return BLASFEO_B200_EINVAL;
 	if (N > 0 && (((uintptr_t)sBA->pA & 15) || ((sBA->stride * sizeof(T)) & 15))) return BLASFEO_B200_EINVAL;
-	if (info) cudaMemsetAsync(info, 0, sizeof(int) * batch, (cudaStream_t)stream);
 	sL->use_dA = 0;
-	const RicLayout<T> lay = ric_layout<T>(nx);
-	const size_t smem = (size_t)lay.warp_bytes * RIC_WARPS;
-	cudaFuncSetAttribute(k_ric_trf<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-	int per_sm = 0;
-	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ric_trf<T>, RIC_WARPS * 32, smem);
-	if (per_sm < 1) per_sm = 1;
-	long long grid = (long long)bf::num_sms() * per_sm;
-	const long long need = (batch + RIC_WARPS - 1) / RIC_WARPS;
-	if (grid > need) grid = need;
-	k_ric_trf<T><<<(unsigned)grid, RIC_WARPS * 32, smem, (cudaStream_t)stream>>>(
-	    batch, N, nx, nu, N > 0 ? sBA->pA : nullptr, N > 0 ? sBA->stride : 0, sRSQ->pA, sRSQ->stride, sL->pA, sL->dA,
-	    sL->stride, info, bf::wait_limit());
-	return bf::check_launch();
+	return ric_launch(batch, N, nx, nu, sBA, sRSQ, sL, info, (cudaStream_t)stream);
 }
 
 }  // namespace

@@ -1,7 +1,7 @@
 // Batched Riccati solve (LQR forward/backward substitution), feedback gains,
 // and the mixed-precision LQ solve: FP32 factorization + FP64 iterative
-// refinement on the KKT residual.  One warp per problem; lane i owns entry i
-// of the stage vectors (nu + nx <= 16).
+// refinement on the KKT residual.  Lane i of a half-warp (FP64 solve, gains) or
+// warp (refinement) owns entry i of a problem's stage vectors (nu + nx <= 16).
 //
 // Problem (examples/example_d_riccati_recursion.c), stages k = 0..N-1 with
 // [u;x]_k of size nu + nx, stage N with x_N only:
@@ -26,7 +26,7 @@
 // dtrsv recomputes its inverse diagonal from the factor).
 #include <math.h>
 
-#include "common.cuh"
+#include "quad.cuh"
 
 namespace {
 
@@ -176,47 +176,274 @@ __device__ void ric_trs_one(const SvArgs &a, long long p, double *sm, int lane) 
 	}
 }
 
-template <typename TL>
-__global__ void __launch_bounds__(SV_WARPS * 32) k_ric_trs(SvArgs a) {
-	extern __shared__ __align__(16) double sv_smem[];
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	double *sm = sv_smem + (size_t)warp * SV_WARP_DBL;
-	const long long nw = (long long)gridDim.x * SV_WARPS;
-	for (long long p = (long long)blockIdx.x * SV_WARPS + warp; p < a.batch; p += nw) ric_trs_one<TL>(a, p, sm, lane);
+// ---- FP64 solve: two problems per warp, stage blocks prefetched ----
+//
+// Lane i of a half-warp owns entry i of its problem's stage vectors (the whole
+// operation order is ric_trs_one's).  Each stage's factor (lower 4 x 4 tiles)
+// and BAbt arrive by cp.async one stage ahead, and the stage's vectors one
+// stage ahead in registers, so the recursion waits for its own chain only;
+// P_k b_{k-1} (backward) and pi_{k-1} (forward) are formed at stage k, where
+// the factor they need is on chip anyway: each sweep reads every factor once.
+// Bound: HBM (both sweeps read L and BAbt; 4,096 problems of 12 + 4 at N = 30
+// hold 346 MB, above L2).  A warp per problem with synchronous block loads
+// took 0.45 ms there, this kernel 0.18.
+constexpr int TRS_WARPS = 2;    // warps per CTA (4 problems: 7 CTAs per SM by shared memory)
+constexpr int TL = 18;          // column stride of the blocks: even for the 16-byte copies
+constexpr int TL2 = 10;         // columns 8..15 of L: rows 8..15 only
+constexpr int TRS_L = 8 * TL + 8 * TL2;
+// doubles per problem: two factors, two BAbt, two vectors
+__host__ __device__ constexpr int trs_el(int nxp) { return 2 * TRS_L + 2 * nxp * TL + 32; }
+
+// start of column c of L in the compact block, minus its row origin
+__device__ __forceinline__ int tcol(int c) { return c < 8 ? c * TL : 8 * TL + (c - 8) * TL2 - 8; }
+__device__ __forceinline__ double shh(double v, int src) { return __shfl_sync(FULL, v, src, 16); }
+
+template <bool VEC>
+__device__ __forceinline__ void cp_pair(double *dst, const double *src) {
+	const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+	if (VEC) {
+		asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+	} else {  // slabs off the 16-byte grid
+		asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+		asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + 8), "l"(src + 1) : "memory");
+	}
 }
 
-// K_k = -Luu^{-T} Lxu^T (nu x nx) from L_k: lane nu + j solves for column j
-__global__ void __launch_bounds__(SV_WARPS * 32)
-    k_ric_gains(int batch, int N, int nx, int nu, const double *pL, long long sl, double *pK, long long sk, int cnk) {
+// lower tiles of a 16 x 16 factor by a half-warp
+template <bool VEC>
+__device__ __forceinline__ void cp_factor(double *dst, const double *L, int i) {
+#pragma unroll
+	for (int it = 0; it < 5; it++) {
+		const int c = 16 * it + i;
+		const int p = c < 8 ? 0 : (c < 24 ? 1 : (c < 48 ? 2 : 3));
+		const int w = c - (p == 0 ? 0 : (p == 1 ? 8 : (p == 2 ? 24 : 48)));
+		cp_pair<VEC>(dst + tcol(w >> 1) + 4 * p + 2 * (w & 1), L + 64 * p + 2 * w);
+	}
+}
+// 16 x NXP block (NXP: nx rounded up to 4), column-major with stride TL
+template <int NXP, bool VEC>
+__device__ __forceinline__ void cp_ba(double *dst, const double *B, int cn, int i) {
+	const int p = (i & 7) >> 1, h = i & 1;
+	const double *g = B + 4 * p * cn + 2 * h;
+	double *d = dst + 4 * p + 2 * h;
+#pragma unroll
+	for (int j = 0; j < NXP; j += 2) cp_pair<VEC>(d + (j + (i >> 3)) * TL, g + 4 * (j + (i >> 3)));
+}
+
+// Entry i of L(o:o+nx, o:o+nx) L(..)^T x for the half-warp's lane i < nx.  x
+// in lanes 0..nx-1; vectors are read back from shared memory two entries at a
+// time (half the instructions of shuffles).  NXP: nx rounded up to 4.
+template <int NXP>
+__device__ __forceinline__ double llt(const double *M, double *xs, int o, int nx, double x, int i) {
+	xs[i] = x;
+	__syncwarp();
+	const double *cb = M + tcol((o + i) & 15) + o;
+	double t = 0.0, z = 0.0;
+#pragma unroll
+	for (int r = 0; r < NXP; r += 2) {
+		const double2 v = *(const double2 *)(xs + r);
+		if (r >= i && r < nx) t = fma(cb[r], v.x, t);
+		if (r + 1 >= i && r + 1 < nx) t = fma(cb[r + 1], v.y, t);
+	}
+	xs[16 + i] = t;
+	__syncwarp();
+	const double *rb = M + tcol(o) + o + i;
+#pragma unroll
+	for (int j = 0; j < NXP; j += 2) {
+		const double2 v = *(const double2 *)(xs + 16 + j);
+		if (j <= i && i < nx) z = fma(*rb, v.x, z);
+		rb += o + j < 7 ? TL : TL2;
+		if (j + 1 <= i && i < nx) z = fma(*rb, v.y, z);
+		rb += o + j + 1 < 7 ? TL : TL2;
+	}
+	return z;
+}
+
+template <int NXP, bool VEC>
+__global__ void __launch_bounds__(TRS_WARPS * 32) k_ric_trs(SvArgs a) {
 	extern __shared__ __align__(16) double sv_smem[];
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	double *Ls = sv_smem + (size_t)warp * RV * LD;
-	const long long nw = (long long)gridDim.x * SV_WARPS;
-	const long long total = (long long)batch * N;
-	for (long long s = (long long)blockIdx.x * SV_WARPS + warp; s < total; s += nw) {
-		const long long p = s / N, k = s % N;
-		ld_block(Ls, pL + sl * (p * (N + 1) + k), RV, RV, lane);
-		const int j = lane - nu;
-		if (j >= 0 && j < nx) {
-			double kc[RV];
+	const int lane = threadIdx.x & 31, i = lane & 15;
+	const int N = a.N, nx = a.nx, nu = a.nu, M = nu + nx;
+	const long long pr = ((long long)blockIdx.x * TRS_WARPS * 2) + (threadIdx.x >> 4);
+	const bool act = pr < a.batch;
+	const long long p = act ? pr : a.batch - 1;  // an idle half works along and stores nothing
+	double *sm = sv_smem + (size_t)(threadIdx.x >> 4) * trs_el(NXP);
+	double *xs = sm + 2 * TRS_L + 2 * NXP * TL;  // 32 entries: vectors shared within the half-warp
+	auto Lb = [&](int k) { return sm + (k & 1) * TRS_L; };
+	auto Bb = [&](int k) { return sm + 2 * TRS_L + (k & 1) * NXP * TL; };
+	const double *gL = (const double *)a.L + a.sl * (p * (N + 1));
+	const double *gB = a.BA + a.sba * (p * N);
+	const double *gb = a.b + a.sb * (p * N) + i;
+	const double *grq = a.rq + a.srq * (p * (N + 1)) + i;
+	double *gux = a.ux + a.sux * (p * (N + 1)) + i;
+	double *gpi = a.pi + a.spi * (p * N) + i;
+	const bool ix = i < nx, im = i < M;
+
+	// ---- backward: stage k in buffer k & 1 ----
+	cp_factor<VEC>(Lb(N), gL + a.sl * N, i);
+	quad::cpa_commit();
+	cp_factor<VEC>(Lb(N - 1), gL + a.sl * (N - 1), i);
+	cp_ba<NXP, VEC>(Bb(N - 1), gB + a.sba * (N - 1), a.cnba, i);
+	quad::cpa_commit();
+	double xn = ix ? grq[a.srq * N] : 0.0;  // x part of ux_{k+1}
+	if (act && ix) gux[a.sux * N] = xn;
+	double rqk = im ? grq[a.srq * (N - 1)] : 0.0;
+	double bk = ix ? gb[a.sb * (N - 1)] : 0.0;
+	asm volatile("cp.async.wait_group 1;" ::: "memory");
+	__syncwarp();
+	double pb = llt<NXP>(Lb(N), xs, 0, nx, bk, i);
+	__syncwarp();
+	for (int k = N - 1; k >= 0; k--) {
+		const double *Lk = Lb(k), *Bk = Bb(k);
+		double rq_next = 0.0, b_next = 0.0;
+		if (k > 0) {
+			cp_factor<VEC>(Lb(k - 1), gL + a.sl * (k - 1), i);
+			cp_ba<NXP, VEC>(Bb(k - 1), gB + a.sba * (k - 1), a.cnba, i);
+			rq_next = im ? grq[a.srq * (k - 1)] : 0.0;
+			b_next = ix ? gb[a.sb * (k - 1)] : 0.0;
+		}
+		quad::cpa_commit();
+		asm volatile("cp.async.wait_group 1;" ::: "memory");
+		xs[i] = ix ? pb + xn : 0.0;
+		__syncwarp();
+		double u = rqk;
+		const double inv = im ? 1.0 / Lk[tcol(i) + i] : 0.0;
 #pragma unroll
-			for (int i = RV - 1; i >= 0; i--) {
-				double c = 0.0;
-				if (i < nu) {
-					c = -Ls[(nu + j) * LD + i];
-#pragma unroll
-					for (int l = i + 1; l < RV; l++)
-						if (l < nu) c = fma(-Ls[l * LD + i], kc[l], c);
-					c *= 1.0 / Ls[i * LD + i];
-				}
-				kc[i] = c;
+		for (int j = 0; j < NXP; j += 2) {
+			const double2 v = *(const double2 *)(xs + j);
+			if (j < nx) u = fma(Bk[j * TL + i], v.x, u);
+			if (j + 1 < nx) u = fma(Bk[(j + 1) * TL + i], v.y, u);
+		}
+		const int ns = k > 0 ? nu : M;
+		const double *rb = Lk + i;
+		for (int j = 0; j < ns; j++) {
+			const double zj = shh(u, j) * shh(inv, j);
+			if (i == j) u = zj;
+			if (i > j && im) u = fma(-rb[0], zj, u);
+			rb += j < 7 ? TL : TL2;
+		}
+		if (act && im) gux[a.sux * k] = u;
+		xn = shh(u, (nu + i) & 15);
+		__syncwarp();
+		if (k > 0) pb = llt<NXP>(Lk, xs, nu, nx, b_next, i);
+		rqk = rq_next;
+		__syncwarp();
+	}
+	// ---- forward: the factor and BAbt of stage 0 are still in buffer 0 ----
+	double xk = 0.0;                        // x_k, lanes 0..nx-1
+	double v = im ? gux[0] : 0.0;           // ux_k of the backward sweep (this lane wrote it)
+	bk = ix ? gb[0] : 0.0;
+	for (int k = 0; k <= N; k++) {
+		const double *Lk = Lb(k), *Bk = Bb(k);
+		double v_next = 0.0, b_next = 0.0;
+		if (k < N) {
+			cp_factor<VEC>(Lb(k + 1), gL + a.sl * (k + 1), i);
+			if (k + 1 < N) {
+				cp_ba<NXP, VEC>(Bb(k + 1), gB + a.sba * (k + 1), a.cnba, i);
+				b_next = ix ? gb[a.sb * (k + 1)] : 0.0;
 			}
+			v_next = (k + 1 < N ? im : ix) ? gux[a.sux * (k + 1)] : 0.0;
+		}
+		quad::cpa_commit();
+		asm volatile("cp.async.wait_group 1;" ::: "memory");
+		__syncwarp();
+		const int o = k < N ? nu : 0;
+		const double pk = shh(v, (o + i) & 15);  // x part of ux_k, backward
+		const double xp = xk;
+		if (k < N) {
+			const double inv = im ? 1.0 / Lk[tcol(i) + i] : 0.0;
+			const double xm = shh(xk, (i - nu) & 15);
+			double u = (k == 0 || i < nu) ? -v : xm;
+			const int ns = k == 0 ? M : nu;
+			const double *cb = Lk + tcol(i);
+			for (int l = M - 1; l >= ns; l--) {
+				const double zl = shh(u, l);
+				if (i < ns) u = fma(-cb[l], zl, u);
+			}
+			for (int l = ns - 1; l >= 0; l--) {
+				const double zl = shh(u, l) * shh(inv, l);
+				if (i == l) u = zl;
+				if (i < l) u = fma(-cb[l], zl, u);
+			}
+			if (act && im) gux[a.sux * k] = u;
+			xs[i] = u;
+			__syncwarp();
+			double x1 = bk;
+			const double *bc = Bk + (ix ? i * TL : 0);
+#pragma unroll
+			for (int l = 0; l < 16; l += 2) {
+				if (l < M) {
+					const double2 ul = *(const double2 *)(xs + l);
+					const double2 bl = *(const double2 *)(bc + l);
+					x1 = fma(bl.x, ul.x, x1);
+					if (l + 1 < M) x1 = fma(bl.y, ul.y, x1);
+				}
+			}
+			xk = x1;
+			__syncwarp();
+		} else if (act && ix) {
+			gux[a.sux * N] = xk;
+		}
+		if (k > 0) {
+			const double w = llt<NXP>(Lk, xs, o, nx, xp, i);
+			if (act && ix) gpi[a.spi * (k - 1)] = pk + w;
+		}
+		v = v_next;
+		bk = b_next;
+		__syncwarp();
+	}
+}
+
+template <bool VEC>
+void launch_trs(const SvArgs &a, cudaStream_t s) {
+	const int q = (a.nx + 3) / 4;
+	auto kern = q == 1 ? k_ric_trs<4, VEC> : (q == 2 ? k_ric_trs<8, VEC> : (q == 3 ? k_ric_trs<12, VEC> : k_ric_trs<16, VEC>));
+	const size_t smem = (size_t)TRS_WARPS * 2 * trs_el(4 * q) * sizeof(double);
+	bf::smem_optin(kern, smem);
+	kern<<<(a.batch + 2 * TRS_WARPS - 1) / (2 * TRS_WARPS), TRS_WARPS * 32, smem, s>>>(a);
+}
+
+// K_k = -Luu^{-T} Lxu^T (nu x nx) from L_k, a half-warp per stage: lane i
+// holds row i of the first nu columns in registers, rows of Luu reach the
+// others by shuffles, lane nu + j solves for column j.  Bound: HBM (nu columns
+// of L in, K out); reading the whole block through shared memory with a
+// division per pivot and lane took 0.113 ms for 122,880 stages of 12 + 4, this
+// kernel 0.028 ms.
+template <int NU>  // nu <= NU
+__global__ void __launch_bounds__(256)
+    k_ric_gains(int batch, int N, int nx, int nu, const double *pL, long long sl, double *pK, long long sk, int cnk) {
+	const int i = threadIdx.x & 15;
+	const long long total = (long long)batch * N;
+	const long long step = (long long)gridDim.x * 16;
+	// both halves of a warp run the same number of steps
+	for (long long s0 = (long long)blockIdx.x * 16 + (threadIdx.x >> 5) * 2; s0 < total; s0 += step) {
+		const long long s1 = s0 + ((threadIdx.x >> 4) & 1);
+		const bool act = s1 < total;
+		const long long s = act ? s1 : total - 1;
+		const long long p = total <= 0x7fffffffLL ? (long long)((unsigned)s / (unsigned)N) : s / N, k = s - p * N;
+		const double *L = pL + sl * (p * (N + 1) + k);
+		double l[NU];
+#pragma unroll
+		for (int c = 0; c < NU; c++) l[c] = (c < nu && c <= i && i < nu + nx) ? L[pmi(i, c, RV)] : 0.0;
+		const double inv = i < nu ? 1.0 / L[pmi(i, i, RV)] : 0.0;
+		double kc[NU];
+#pragma unroll
+		for (int r = NU - 1; r >= 0; r--) {
+			double c = -l[r];
+#pragma unroll
+			for (int q = r + 1; q < NU; q++) {
+				const double lqr = shh(l[r], q);
+				if (q < nu) c = fma(-lqr, kc[q], c);
+			}
+			kc[r] = c * shh(inv, r);
+		}
+		const int j = i - nu;
+		if (act && j >= 0 && j < nx) {
 			double *g = pK + sk * s;
 #pragma unroll
-			for (int i = 0; i < RV; i++)
-				if (i < nu) g[pmi(i, j, cnk)] = kc[i];
+			for (int r = 0; r < NU; r++)
+				if (r < nu) g[pmi(r, j, cnk)] = kc[r];
 		}
-		__syncwarp();
 	}
 }
 
@@ -388,9 +615,10 @@ int blasfeo_dric_trs_batch(int batch, int N, int nx, int nu, struct blasfeo_dmat
 	if (batch == 0) return BLASFEO_B200_OK;
 	SvArgs a{batch, N, nx, nu, sBAbt->pA, sBAbt->stride, sBAbt->cn, sL->pA, sL->stride, b, sb, rq, srq,
 	         ux, sux, pi, spi};
-	const size_t smem = (size_t)SV_WARP_DBL * SV_WARPS * sizeof(double);
-	k_ric_trs<double><<<grid_of(batch, smem, (const void *)k_ric_trs<double>), SV_WARPS * 32, smem,
-	                    (cudaStream_t)stream>>>(a);
+	if ((((uintptr_t)a.BA | (uintptr_t)a.L) & 15) || ((a.sba | a.sl) & 1))
+		launch_trs<false>(a, (cudaStream_t)stream);
+	else
+		launch_trs<true>(a, (cudaStream_t)stream);
 	return bf::check_launch();
 }
 
@@ -402,9 +630,11 @@ int blasfeo_dric_gains_batch(int batch, int N, int nx, int nu, struct blasfeo_dm
 		return BLASFEO_B200_EINVAL;
 	if (batch == 0) return BLASFEO_B200_OK;
 	sK->use_dA = 0;
-	const size_t smem = (size_t)RV * LD * SV_WARPS * sizeof(double);
-	k_ric_gains<<<grid_of((long long)batch * N, smem, (const void *)k_ric_gains), SV_WARPS * 32, smem,
-	              (cudaStream_t)stream>>>(batch, N, nx, nu, sL->pA, sL->stride, sK->pA, sK->stride, sK->cn);
+	// registers by the number of inputs; 8 half-warp pairs per CTA, the grid capped at full residency
+	auto kern = nu <= 4 ? k_ric_gains<4> : (nu <= 8 ? k_ric_gains<8> : k_ric_gains<16>);
+	const long long need = ((long long)batch * N + 15) / 16, cap = 8LL * bf::num_sms();
+	kern<<<(unsigned)(need < cap ? need : cap), 256, 0, (cudaStream_t)stream>>>(batch, N, nx, nu, sL->pA, sL->stride,
+	                                                                             sK->pA, sK->stride, sK->cn);
 	return bf::check_launch();
 }
 

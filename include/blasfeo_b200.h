@@ -133,7 +133,7 @@ int blasfeo_b200_version(void);
  * the roofline denominator of the SIMT kernels (no reference counterpart) */
 double blasfeo_b200_measure_fma_peak(char prec, int iters);
 /* Polls of every bounded mbarrier wait of the kernels that use bulk copies
- * (the fused n=16 chain, the batched Riccati factorization, the tensor-memory
+ * (the fused n=16 chain, the FP32 batched Riccati factorization, the tensor-memory
  * engine of the mixed solver), process-wide; 0 restores the default (2^24
  * polls, about one second).  A wait that runs out sets the instance's
  * info = -3 and the kernel returns after draining its copies (no reference
@@ -530,7 +530,8 @@ int blasfeo_dsyrk_dpotrf_dtrsm_dgemm_batch(int batch, int m, int k, double shift
  * batch*(N+1) instances of 16 x 16 (problem b, stage k at b*(N+1) + k; stage N
  * holds Q_N / L_N in its top-left nx x nx block).  Outputs: L_k (lower
  * triangle) and its inverse diagonal in sL's dA; info[b] = 16*(N-k) + j + 1
- * for the first non-positive pivot j of stage k, -3 on a copy timeout. */
+ * for the first non-positive pivot j of stage k (sric only: -3 on a copy
+ * timeout). */
 int blasfeo_dric_trf_batch(int batch, int N, int nx, int nu, struct blasfeo_dmat_batch *sBAbt,
 	struct blasfeo_dmat_batch *sRSQ, struct blasfeo_dmat_batch *sL, int *info, void *stream);
 int blasfeo_sric_trf_batch(int batch, int N, int nx, int nu, struct blasfeo_smat_batch *sBAbt,
