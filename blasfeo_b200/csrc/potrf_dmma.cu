@@ -6,35 +6,28 @@
 // m8n8 accumulator fragment: lane l keeps row 8I + l/4, columns 8J + 2(l%4)
 // and 8J + 2(l%4) + 1.  Unfactored blocks are kept NEGATED (F = -A), so the
 // rank-8 trailing update A_IJ -= L_IK L_JK^T is a plain accumulate,
-// F_IJ += L_IK L_JK^T, two m8n8k4 DMMAs per block.  Both operand fragments of
-// that product (8 rows x 4 k, lane l: row l/4, k l%4) are the same shuffle of
-// the factored panel block, so one fragment pair per block row serves as A
-// and as B.
+// F_IJ += L_IK L_JK^T, two m8n8k4 DMMAs per block.
 //
-// Right-looking by 8-column panels K:
-//   panel:   column by column, the FP64 pivot is broadcast by a shuffle, its
-//            reciprocal square root taken (pivot rule of
-//            kernel/generic/kernel_dgemm_4x4_lib4.c:5700-5710: c > 0 ->
-//            L_jj = c * rsqrt(c), dA_j = rsqrt(c); else 0 and 0), the column
-//            scaled and the rest of the panel updated with FMAs;
-//   trailing: every block right of the panel, two DMMAs each.
-// Everything is unrolled over the compile-time block grid (N8 = ceil(n/8)), so
-// the fragments never leave registers; rows and columns n..8*N8-1 hold the
-// identity.  The instance arrives through shared memory (16-byte cp.async
-// copies of the lower panels, all in flight together).  HBM traffic: one read
-// and one write of the lower triangle.
-#include "common.cuh"
+// Right-looking by 8-column panels (chol_frag.cuh): the panel's pivots two at
+// a time, then every block right of it gets two DMMAs.  Pivot rule of
+// kernel/generic/kernel_dgemm_4x4_lib4.c:5700-5710: c > 0 -> L_jj = c * rsqrt(c),
+// dA_j = rsqrt(c); else 0 and 0.  Everything is unrolled over the compile-time
+// block grid (N8 = ceil(n/8)), so the fragments never leave registers; rows and
+// columns n..8*N8-1 hold the identity.  The instance arrives through shared
+// memory (16-byte cp.async copies of the lower panels, all in flight
+// together).  HBM traffic: one read and one write of the lower triangle.
+//
+// Bound: the pivot chain (two pivots per 220 cycles) with the warps that the
+// registers allow (8 per SM at n = 64), then the FP64 tensor pipe (384 steps of
+// 15 cycles per SM sub-partition at n = 64).  8,000 matrices of n = 64: pivots,
+// rows and columns broadcast by shuffles 171 us, this form 155 us (n = 48:
+// 21,000 matrices 526 -> 309 us, n = 32: 40,000 198 -> 150 us).
+#include "chol_frag.cuh"
 #include "kernels.cuh"
 
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
-
-__device__ __forceinline__ void dmma_acc(double &d0, double &d1, double a, double b) {
-	asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-	             : "+d"(d0), "+d"(d1)
-	             : "d"(a), "d"(b));
-}
 
 __host__ __device__ constexpr int blk(int i, int j) { return i * (i + 1) / 2 + j; }
 
@@ -46,6 +39,63 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
 // columns 0..4p+3 at offset 8p(p+1), the global panel layout cut at the
 // diagonal tile)
 __host__ __device__ constexpr int lower_panels(int n8) { return 8 * (n8 / 4) * (n8 / 4 + 1); }
+
+// shared memory of one warp: the lower panels, then 64 inverse pivots and the
+// 16 entries of frag::panel
+__host__ __device__ constexpr int warp_doubles(int n8) { return lower_panels(8 * n8) + 80; }
+
+// The same factorization column by column in global memory by one warp, for
+// matrices with a pivot that chol_rsqrt does not take (subnormal or infinite)
+__device__ __noinline__ void potrf_warp(PMat<double> c, PMat<double> d, int n, int *info, int lane) {
+	int bad = 0;
+	for (int j = 0; j < n; j++)
+		for (int i = j + lane; i < n; i += 32) d.at(i, j) = c.at(i, j);
+	__syncwarp();
+	for (int j = 0; j < n; j++) {
+		const double p = d.at(j, j);
+		const bool ok = p > 0.0;
+		const double iv = ok ? rsqrt(p) : 0.0;
+		if (!ok && bad == 0) bad = j + 1;
+		__syncwarp();
+		for (int i = j + lane; i < n; i += 32) d.at(i, j) = (i == j && !ok) ? 0.0 : d.at(i, j) * iv;
+		if (lane == 0) d.d[j] = iv;
+		__syncwarp();
+		for (int l = j + 1; l < n; l++) {
+			const double t = d.at(l, j);
+			for (int i = l + lane; i < n; i += 32) d.at(i, l) = fma(-d.at(i, j), t, d.at(i, l));
+		}
+		__syncwarp();
+	}
+	if (info && lane == 0) *info = bad;
+}
+
+// panels K.. of the factorization (compile-time K, so the fragments stay in registers)
+template <int N8, int K>
+__device__ __forceinline__ void factor(double (&F)[N8 * (N8 + 1) / 2][2], double *sc, double *dv, int r, int q) {
+	if constexpr (K < N8) {
+		double P[N8 - K][2];
+#pragma unroll
+		for (int I = K; I < N8; I++) {
+			P[I - K][0] = F[blk(I, K)][0];
+			P[I - K][1] = F[blk(I, K)][1];
+		}
+		frag::panel<N8 - K, true>(P, sc, dv + 8 * K, r, q);
+		// trailing update, next panel's column first, the first step of every
+		// block of a column before the second
+#pragma unroll
+		for (int J = K + 1; J < N8; J++)
+#pragma unroll
+			for (int e = 0; e < 2; e++)
+#pragma unroll
+				for (int I = J; I < N8; I++) frag::dmma(F[blk(I, J)][0], F[blk(I, J)][1], P[I - K][e], P[J - K][e]);
+#pragma unroll
+		for (int I = K; I < N8; I++) {
+			F[blk(I, K)][0] = P[I - K][0];
+			F[blk(I, K)][1] = P[I - K][1];
+		}
+		factor<N8, K + 1>(F, sc, dv, r, q);
+	}
+}
 
 template <int N8, int WPC, int MINB>
 __global__ void __launch_bounds__(32 * WPC, MINB) k_potrf_dmma(int batch, SizeArg sz, MatArg<double> C,
@@ -64,7 +114,8 @@ __global__ void __launch_bounds__(32 * WPC, MINB) k_potrf_dmma(int batch, SizeAr
 	// fill the fragments from there.  Rows not starting a panel, or panels not
 	// 16-byte aligned, are read element by element from global memory.
 	extern __shared__ __align__(16) double pot_smem[];
-	double *S = pot_smem + (threadIdx.x >> 5) * lower_panels(8 * N8);
+	double *S = pot_smem + (threadIdx.x >> 5) * warp_doubles(N8);
+	double *dv = S + lower_panels(8 * N8);
 	const bool staged = ((c.ri & 3) == 0) && ((((uintptr_t)c.p) & 15) == 0);
 	if (staged) {
 		const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(S);
@@ -99,65 +150,24 @@ __global__ void __launch_bounds__(32 * WPC, MINB) k_potrf_dmma(int batch, SizeAr
 				F[blk(I, J)][h] = v;
 			}
 
-	int bad = 0;
+	factor<N8, 0>(F, dv + 64, dv, r, q);
+	__syncwarp();
+	const double i0 = dv[lane], i1 = N8 > 4 ? dv[N8 > 4 ? 32 + lane : 0] : 1.0;
+	const double inf = __longlong_as_double(0x7ff0000000000000LL);
+	if (__any_sync(FULL, (lane < 8 * N8 && !(i0 < inf)) || (32 + lane < 8 * N8 && !(i1 < inf)))) {
+		potrf_warp(c, d, n, info ? info + b : nullptr, lane);
+		return;
+	}
+	if (lane < n) d.d[lane] = i0;
+	if (32 + lane < n) d.d[32 + lane] = i1;
+	const unsigned z0 = __ballot_sync(FULL, lane < n && i0 == 0.0), z1 = __ballot_sync(FULL, 32 + lane < n && i1 == 0.0);
+	const int bad = z0 ? __ffs(z0) : (z1 ? 32 + __ffs(z1) : 0);
+	if (bad) {
 #pragma unroll
-	for (int K = 0; K < N8; K++) {
-		const int KK = blk(K, K);
-		// ---- panel K, column by column ----
+		for (int I = 0; I < N8; I++)
 #pragma unroll
-		for (int cc = 0; cc < 8; cc++) {
-			const int e = cc & 1, src = cc >> 1;
-			const double cv = -__shfl_sync(FULL, F[KK][e], (cc << 2) | src);
-			const bool ok = cv > 0.0;
-			const double inv = ok ? rsqrt(cv) : 0.0;
-			const double lcc = ok ? cv * inv : 0.0;
-			if (!ok && bad == 0) bad = 8 * K + cc + 1;
-			if (lane == 0 && 8 * K + cc < n) d.d[8 * K + cc] = inv;
-			// scale column cc (held by the lanes with q == cc/2, element cc&1)
-			if (q == src) {
-#pragma unroll
-				for (int I = K; I < N8; I++) {
-					double &x = F[blk(I, K)][e];
-					if (I > K || r > cc)
-						x = -x * inv;
-					else if (r == cc)
-						x = lcc;
-				}
-			}
-			if (cc < 7) {
-				// update columns cc+1..7 of the panel: F(i,c') += L(i,cc) L(8K+c',cc)
-				const double lk0 = __shfl_sync(FULL, F[KK][e], ((2 * q) << 2) | src);
-				const double lk1 = __shfl_sync(FULL, F[KK][e], ((2 * q + 1) << 2) | src);
-#pragma unroll
-				for (int I = K; I < N8; I++) {
-					const double li = __shfl_sync(FULL, F[blk(I, K)][e], (lane & ~3) | src);
-					if (2 * q > cc && (I > K || r >= 2 * q)) F[blk(I, K)][0] = fma(li, lk0, F[blk(I, K)][0]);
-					if (2 * q + 1 > cc && (I > K || r >= 2 * q + 1))
-						F[blk(I, K)][1] = fma(li, lk1, F[blk(I, K)][1]);
-				}
-			}
-		}
-		if (K + 1 == N8) continue;
-		// ---- operand fragments of the factored panel: a0 = L(8I+r, 8K+q), a1 = L(8I+r, 8K+4+q) ----
-		double a0[N8], a1[N8];
-#pragma unroll
-		for (int I = K + 1; I < N8; I++) {
-			const int s0 = (lane & ~3) | (q >> 1), s1 = (lane & ~3) | (2 + (q >> 1));
-			const double t00 = __shfl_sync(FULL, F[blk(I, K)][0], s0);
-			const double t01 = __shfl_sync(FULL, F[blk(I, K)][1], s0);
-			const double t10 = __shfl_sync(FULL, F[blk(I, K)][0], s1);
-			const double t11 = __shfl_sync(FULL, F[blk(I, K)][1], s1);
-			a0[I] = (q & 1) ? t01 : t00;
-			a1[I] = (q & 1) ? t11 : t10;
-		}
-		// ---- trailing update, next panel's column first ----
-#pragma unroll
-		for (int J = K + 1; J < N8; J++)
-#pragma unroll
-			for (int I = J; I < N8; I++) {
-				dmma_acc(F[blk(I, J)][0], F[blk(I, J)][1], a0[I], a0[J]);
-				dmma_acc(F[blk(I, J)][0], F[blk(I, J)][1], a1[I], a1[J]);
-			}
+			for (int h = 0; h < 2; h++)
+				if (r == 2 * q + h && dv[8 * I + r] == 0.0) F[blk(I, I)][h] = 0.0;
 	}
 
 	// store the lower triangle of L
@@ -176,11 +186,11 @@ __global__ void __launch_bounds__(32 * WPC, MINB) k_potrf_dmma(int batch, SizeAr
 template <int N8>
 void launch_n8(int batch, SizeArg sz, MatArg<double> C, MatArg<double> D, int *info, cudaStream_t s) {
 	constexpr int WPC = N8 <= 4 ? 4 : (N8 <= 6 ? 2 : 1);
-	// n in 49..56: 168 registers (the fragments still fit) for 12 resident
-	// warps per SM instead of 8 (measured 3.7 -> 4.4 TF/s at n = 56); at
-	// n = 64 the same cap spills fragments and loses (4.4 -> 2.9 TF/s)
-	constexpr int MINB = N8 == 7 ? 12 : 1;
-	const size_t smem = (size_t)WPC * lower_panels(8 * N8) * sizeof(double);
+	// resident CTAs per SM by the registers that the fragments need: 8, 12, 16,
+	// 16, 20, 24, 32, 32 warps per SM for N8 = 8 .. 1 (the chain of a matrix is
+	// hidden by the others; a tighter cap spills fragments)
+	constexpr int MINB = N8 == 8 ? 8 : (N8 == 7 ? 12 : (N8 >= 5 ? 8 : (N8 == 4 ? 5 : (N8 == 3 ? 6 : 8))));
+	const size_t smem = (size_t)WPC * warp_doubles(N8) * sizeof(double);
 	k_potrf_dmma<N8, WPC, MINB><<<(batch + WPC - 1) / WPC, 32 * WPC, smem, s>>>(batch, sz, C, D, info);
 }
 
