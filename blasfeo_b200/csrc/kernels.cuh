@@ -24,6 +24,13 @@ int dpotrf_ll_max_n();
 int dpotrf_ll_launch(int batch, SizeArg sz, int min_n, int max_m, MatArg<double> C, MatArg<double> D, int *info,
                      cudaStream_t s);
 
+// FP64 getrf_rp / getrf_np with the panels in registers (getrf_reg.cu): whether
+// it takes matrices up to max_m x max_n, and the launch with nt = 64, 128, 256
+// or 512 threads per matrix (raised where a matrix has more rows than fit)
+bool dgetrf_reg_fits(int max_m, int max_n);
+int dgetrf_reg_launch(int batch, SizeArg sz, MatArg<double> C, MatArg<double> D, int *ipiv, long long stride, int *info,
+                      cudaStream_t s, int max_m, int max_n, bool piv, int nt);
+
 // D = chol(C) lower, inverse diagonal into D's dA, info (device, may be null)
 template <typename T>
 int potrf_launch(int batch, SizeArg sz, int max_m, MatArg<T> C, MatArg<T> D, int *info, cudaStream_t s,

@@ -1277,8 +1277,9 @@ int syrk_potrf_batch(int batch, int m, int k, BT *sA, int ai, int aj, BT *sB, in
 	return bf::potrf_launch<T>(batch, uniform_sizes(m, m, 0), m, D, D, info, s, -1);
 }
 
-// variant: -1 auto; 0..2: the blocked global-memory kernels (getrf: 128
-// threads with 4 or 2 blocks per SM, 256 threads; geqrf: 256 threads with the
+// variant: -1 auto; 0..2: the blocked global-memory kernels (getrf FP64: register
+// panels with 128 / 256 / 512 threads, getrf_reg.cu; FP32: 128 threads with 4
+// or 2 blocks per SM, 256 threads; geqrf: 256 threads with the
 // SIMT trailing update, 256 and 512 threads with the DMMA one); 3..5: the
 // instances whose block fits in shared memory there (128/256/512 threads),
 // the others in the blocked global-memory kernel (a second launch).
@@ -1336,8 +1337,8 @@ inline size_t lu_smem_bytes(int max_m, int max_n, size_t esz) {
 
 // built-in rule for getrf (qr = false) and geqrf (qr = true), from uniform
 // batches timed on the B200 at n = 32..384: the shared-memory kernel with 128
-// threads for small blocks, the blocked global-memory kernels above (getrf:
-// 128 threads with 4 blocks per SM up to n = 96, with 3 up to 288, then 256
+// threads for small blocks, the blocked global-memory kernels above (getrf, FP32:
+// 128 threads with 4 blocks per SM up to n = 96, with 2 up to 288, then 256
 // threads; geqrf: shared memory up to 64 rows, then the DMMA update with
 // 256 threads at 2 CTAs per SM)
 inline int pick_lu_variant(int variant, int max_m, int max_n, bool qr = false) {
@@ -1353,6 +1354,21 @@ inline int pick_lu_variant(int variant, int max_m, int max_n, bool qr = false) {
 	return variant;
 }
 
+// built-in rule for FP64 getrf with register panels, by matrix size, from
+// uniform batches (us; 128 / 256 / 512 threads): n = 128 x 9,251 3,654 / 4,428 /
+// 7,684, n = 160 x 5,662 4,706 / 4,000 / 6,494, n = 256 x 2,013 5,256 / 3,807 /
+// 5,169, n = 320 x 1,232 5,100 (256) / 5,322.  With one or two matrices per SM
+// the largest one sets the time and 512 threads finish it first (1,024 of sizes
+// log-uniform to 384: 1,136 / 741 for 256 / 512; 4,096: 3,621 / 3,961).
+// Uneven launches of a few hundred matrices are of that kind below n = 256 too
+// (600 of sizes to 200: 302 / 254).
+inline int pick_getrf_reg(int batch, int max_m, int max_n, bool uneven) {
+	const int mx = max_m > max_n ? max_m : max_n;
+	if (mx <= 128) return 0;
+	if (mx <= 256) return batch <= (uneven ? 6 : 2) * bf::num_sms() ? 2 : 1;
+	return batch <= 16 * bf::num_sms() ? 2 : 1;
+}
+
 template <typename T>
 int getrf_launch(int batch, SizeArg sz, MatArg<T> C, MatArg<T> D, int *ipiv, long long ipiv_stride, int *info,
                  cudaStream_t s, int max_m, int max_n, int variant = -1, bool piv = true) {
@@ -1360,20 +1376,29 @@ int getrf_launch(int batch, SizeArg sz, MatArg<T> C, MatArg<T> D, int *ipiv, lon
 	const size_t need = lu_smem_bytes(max_m, max_n, sizeof(T));
 	const size_t smem = need < cap_full ? need : cap_full;
 	const int cap = (int)smem;
+	if (sizeof(T) == 8 && variant < 0 && bf::dgetrf_reg_fits(max_m, max_n))
+		variant = pick_getrf_reg(batch, max_m, max_n, sz.pm != nullptr);
 	variant = pick_lu_variant(variant, max_m, max_n);
+	if constexpr (sizeof(T) == 8) {
+		// up to 512 rows: the panel in registers, 128, 256 or 512 threads
+		// (variant 0: 32 or 64 where that covers the rows)
+		if (variant < 3 && bf::dgetrf_reg_fits(max_m, max_n))
+			return bf::dgetrf_reg_launch(batch, sz, C, D, ipiv, ipiv_stride, info, s, max_m, max_n, piv,
+			                             variant > 0 ? 128 << variant : (max_m <= 32 ? 32 : (max_m <= 64 ? 64 : 128)));
+	}
+	if constexpr (sizeof(T) == 8) {
+		// beyond the register panels: blocked in global memory
+		if (variant < 3) variant = 2;
+	}
 	switch (variant) {
-	// blocked: 128 threads with 4 or 3 blocks per SM (register cap; FP64 variant 1
-	// spills a little at 3, faster than 2: n = 224 2.25 -> 2.65 TF/s), 256 threads
-	case 0: launch_getrf_blk<T, 128, 4>(batch, sz, -1, max_m, max_n, C, D, ipiv, ipiv_stride, info, s, piv); break;
+	// blocked (FP32): 128 threads with 4 or 2 blocks per SM (register cap), 256 threads
+	case 0:
+		if constexpr (sizeof(T) == 4)
+			launch_getrf_blk<T, 128, 4>(batch, sz, -1, max_m, max_n, C, D, ipiv, ipiv_stride, info, s, piv);
+		break;
 	case 1:
-		// FP64: 3 CTAs per SM up to n = 288 (the size rule's range), 2 above:
-		// batches that mix sizes up to 384 ran faster with 2 (mixed-op stream,
-		// LU share 348 -> 329 ms)
-		if (sizeof(T) == 8 && (max_m > 288 || max_n > 288))
+		if constexpr (sizeof(T) == 4)
 			launch_getrf_blk<T, 128, 2>(batch, sz, -1, max_m, max_n, C, D, ipiv, ipiv_stride, info, s, piv);
-		else
-			launch_getrf_blk<T, 128, sizeof(T) == 8 ? 3 : 2>(batch, sz, -1, max_m, max_n, C, D, ipiv, ipiv_stride,
-			                                                   info, s, piv);
 		break;
 	case 2: launch_getrf_blk<T, 256, 1>(batch, sz, -1, max_m, max_n, C, D, ipiv, ipiv_stride, info, s, piv); break;
 	case 3: launch_getrf<T, 128, true>(batch, sz, cap, smem, C, D, ipiv, ipiv_stride, info, s, piv); break;
