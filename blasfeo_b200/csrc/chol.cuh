@@ -19,7 +19,7 @@
 //      factored diagonal block (one row per thread, the reciprocal pivots
 //      multiplied in);
 //   B. warp 0 (critical path): rank-16 update of the 16x16 diagonal block K+1
-//      and its factorization in FP64 registers (pivot rule of
+//      and its factorization in FP64 fragments (chol_diag; pivot rule of
 //      kernel/generic/kernel_dgemm_4x4_lib4.c:5700-5710: c>0 -> sqrt(c) and its
 //      reciprocal, else 0 and 0); the warps on the other three schedulers:
 //      rank-16 update of the rest of the trailing matrix (8 x 4 tile blocks
@@ -28,9 +28,8 @@
 // inverses (FP64 arithmetic, all blocks in parallel) for the blocked
 // triangular solves of the factor+solve kernels.
 #pragma once
+#include "chol_frag.cuh"
 #include "common.cuh"
-
-#define CHOL_NB 16
 
 __host__ __device__ __forceinline__ int lp_off(int p) { return 8 * p * (p + 1); }
 __host__ __device__ __forceinline__ int lp_size(int n) {
@@ -118,203 +117,67 @@ __device__ __forceinline__ void chol_pivot_rsqrt(double c, double &d, double &in
 	}
 }
 
-// One column J of the 16x16 diagonal-block factorization; lane i holds row i
-// of the block in r[] (compile-time indices only, so r stays in registers).
-// The pivot is broadcast by a shuffle and every lane computes its reciprocal
-// square root in FP64 (T = float: FP32 entries and updates, FP64 pivots);
-// column J reaches the other rows by shuffles.  The pivot rule is applied
-// without branches so the compiler can overlap the column update with the
-// next pivot.  The terminal step records the first non-positive pivot
-// (c0 + j + 1) in *bad by one ballot over the rows.
-// WIDTH = 16 factors two independent blocks per warp, one per half-warp:
-// `lane` is then the lane within the half (0..15), the shuffles stay inside
-// the half, and each half records its own dinv / bad (the caller passes the
-// half's pointers).  The whole warp executes the call.
-template <int J, typename T = double, int WIDTH = 32>
-struct DiagCol {
-	static __device__ __forceinline__ void run(T (&r)[CHOL_NB], int lane, int nbk, int c0, double *dinv, int *bad) {
-		const double cj = (double)__shfl_sync(0xffffffffu, r[J], J, WIDTH);
-		const bool ok = cj > 0.0;
-		const double inv = ok ? rsqrt(cj) : 0.0;
-		r[J] = (lane == J) ? (T)(ok ? cj * inv : 0.0) : r[J] * (T)inv;
-		if (lane == J && J < nbk) dinv[c0 + J] = inv;
-#pragma unroll
-		for (int l = J + 1; l < CHOL_NB; l++) {
-			const T t = __shfl_sync(0xffffffffu, r[J], l, WIDTH);
-			if (lane >= l) r[l] = fma(-r[J], t, r[l]);
-		}
-		DiagCol<J + 1, T, WIDTH>::run(r, lane, nbk, c0, dinv, bad);
-	}
-};
-template <typename T, int WIDTH>
-struct DiagCol<CHOL_NB, T, WIDTH> {
-	static __device__ __forceinline__ void run(T (&r)[CHOL_NB], int lane, int nbk, int c0, double *, int *bad) {
-		T d = T(1);
-#pragma unroll
-		for (int l = 0; l < CHOL_NB; l++)
-			if (l == lane) d = r[l];
-		unsigned m = __ballot_sync(0xffffffffu, lane < nbk && !(d > T(0)));
-		if (WIDTH == 16) m = (m >> (threadIdx.x & 16)) & 0xffffu;  // this half-warp's rows
-		if (m && lane == 0 && *bad == 0) *bad = c0 + __ffs(m);
-	}
-};
+// Doubles of scratch of the diagonal blocks: the row-major copy Lt (16 x 17,
+// sized for FP64), then what frag::chol16 needs
+constexpr int CHOL_SCR = 16 * 17 + 32;
 
-// FP32 data: the 16 x 16 lower block, staged row-major in blk (16 rows of 17),
-// is factored by every lane of the warp at once, each holding the whole lower
-// triangle in registers, so the pivot chain issues no shuffles: under the
-// trailing update of the other warps, which keeps the shared-memory / shuffle
-// unit busy, each of the 16 pivot steps of DiagCol waited for that unit
-// several times (clock64 probe of the n = 256 solver: 11.7k cycles per block).
-// Same operations in the same order as DiagCol (pivot rule of
-// kernel/generic/kernel_dgemm_4x4_lib4.c:5700-5710 with FP64 pivots and
-// reciprocals, column scaling, then the rank-1 update of the trailing columns
-// in column order), so the factor is bitwise the same.  Lane i < 16 receives
-// row i of L in r; lane i < nbk writes dinv[c0 + i]; the first non-positive
-// pivot (c0 + j + 1) goes to *bad.
+// Warp 0: the diagonal block at column c0n (nbk <= 16 real columns; the
+// padding is the identity), in FP64 tensor core fragments whatever T is.
+// c0 >= 0 (look-ahead step): first its rank-16 update with the panel of block
+// column c0 (already solved).  Writes L_KK back into S, 1/L_jj into
+// dinv[c0n + j] (FP64), the first bad pivot (c0n + j + 1) into *bad, and for
+// the panel solve a row-major 16x17 copy Lt of L_KK in the working precision
+// with the reciprocal pivots in column 16.  This block is the critical path of
+// the factorization; with a row per lane and shuffles it waited for the
+// shared-memory / shuffle unit that the update warps keep busy (n = 256, FP32:
+// 11.7k cycles per block beside a full trailing update).
 template <typename T>
-__device__ __forceinline__ void diag_factor_rep(const T *blk, int nbk, int c0, double *dinv, int *bad,
-                                                T (&r)[CHOL_NB], int lane) {
-	T a[CHOL_NB * (CHOL_NB + 1) / 2];  // packed lower triangle, (i, j) at i (i + 1) / 2 + j
+__device__ void chol_diag(T *S, int c0n, int nbk, int c0, double *dinv, T *Lt, int *bad) {
+	const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+	double *scr = (double *)Lt + 16 * 17;
+	double F[3][2];
 #pragma unroll
-	for (int i = 0; i < CHOL_NB; i++)
-#pragma unroll
-		for (int j = 0; j <= i; j++) a[i * (i + 1) / 2 + j] = blk[i * 17 + j];
-	double inv_all[CHOL_NB];
-	int first_bad = 0;
-#pragma unroll
-	for (int J = 0; J < CHOL_NB; J++) {
-		const double cj = (double)a[J * (J + 1) / 2 + J];
-		const bool ok = cj > 0.0;
-		const double inv = ok ? rsqrt(cj) : 0.0;
-		inv_all[J] = inv;
-		if (!ok && J < nbk && first_bad == 0) first_bad = J + 1;
-		a[J * (J + 1) / 2 + J] = (T)(ok ? cj * inv : 0.0);
-#pragma unroll
-		for (int i = J + 1; i < CHOL_NB; i++) a[i * (i + 1) / 2 + J] = a[i * (i + 1) / 2 + J] * (T)inv;
-#pragma unroll
-		for (int l = J + 1; l < CHOL_NB; l++)
-#pragma unroll
-			for (int i = l; i < CHOL_NB; i++)
-				a[i * (i + 1) / 2 + l] = fma(-a[i * (i + 1) / 2 + J], a[l * (l + 1) / 2 + J], a[i * (i + 1) / 2 + l]);
+	for (int h = 0; h < 2; h++) {
+		const int j = 2 * q + h;
+		const bool r0 = g < nbk, r1 = 8 + g < nbk;
+		F[0][h] = r0 ? (j <= g ? -(double)lp_at(S, c0n + g, c0n + j) : 0.0) : (j == g ? -1.0 : 0.0);
+		F[1][h] = r1 ? -(double)lp_at(S, c0n + 8 + g, c0n + j) : 0.0;
+		F[2][h] = r1 ? (j <= g ? -(double)lp_at(S, c0n + 8 + g, c0n + 8 + j) : 0.0) : (j == g ? -1.0 : 0.0);
 	}
+	if (c0 >= 0) {
+		double a0[4], a1[4];
 #pragma unroll
-	for (int l = 0; l < CHOL_NB; l++) r[l] = T(0);
-#pragma unroll
-	for (int i = 0; i < CHOL_NB; i++)
-		if (lane == i) {
-#pragma unroll
-			for (int l = 0; l <= i; l++) r[l] = a[i * (i + 1) / 2 + l];
-			if (i < nbk) dinv[c0 + i] = inv_all[i];
+		for (int ks = 0; ks < 4; ks++) {
+			a0[ks] = g < nbk ? (double)lp_at(S, c0n + g, c0 + 4 * ks + q) : 0.0;
+			a1[ks] = 8 + g < nbk ? (double)lp_at(S, c0n + 8 + g, c0 + 4 * ks + q) : 0.0;
 		}
-	if (lane == 0 && first_bad && *bad == 0) *bad = c0 + first_bad;
-}
-
-// Write the factored diagonal block (lane i: row i in r) back into S and into
-// the row-major Lt (reciprocal pivots, from the FP64 dinv, in column 16).
-template <typename T>
-__device__ __forceinline__ void chol_diag_store(T *S, int c0, int nbk, const double *dinv, T *Lt, const T (&r)[CHOL_NB],
-                                                int lane) {
-	if (lane < CHOL_NB) {
 #pragma unroll
-		for (int l = 0; l < CHOL_NB; l++) Lt[lane * 17 + l] = (l <= lane) ? r[l] : T(0);
-		if (lane < nbk) {
+		for (int ks = 0; ks < 4; ks++) {
+			frag::dmma(F[0][0], F[0][1], a0[ks], a0[ks]);
+			frag::dmma(F[1][0], F[1][1], a1[ks], a0[ks]);
+			frag::dmma(F[2][0], F[2][1], a1[ks], a1[ks]);
+		}
+	}
+	const double v = frag::chol16(F, scr, lane);
+	const unsigned m = __ballot_sync(0xffffffffu, lane < nbk && frag::bad_pivot(v));
+	if (m && lane == 0 && *bad == 0) *bad = c0n + __ffs(m);
+	if (lane < nbk) dinv[c0n + lane] = fabs(v);
+	if (lane < 16) Lt[lane * 17 + 16] = (T)fabs(v);
 #pragma unroll
-			for (int l = 0; l < CHOL_NB; l++)
-				if (l <= lane) lp_at(S, c0 + lane, c0 + l) = r[l];
+	for (int h = 0; h < 2; h++) {
+		const int j = 2 * q + h;
+		const T l0 = j <= g ? (T)F[0][h] : T(0), l1 = (T)F[1][h], l2 = j <= g ? (T)F[2][h] : T(0);
+		Lt[g * 17 + j] = l0;
+		Lt[g * 17 + 8 + j] = T(0);
+		Lt[(8 + g) * 17 + j] = l1;
+		Lt[(8 + g) * 17 + 8 + j] = l2;
+		if (g < nbk && j <= g) lp_at(S, c0n + g, c0n + j) = l0;
+		if (8 + g < nbk) {
+			lp_at(S, c0n + 8 + g, c0n + j) = l1;
+			if (j <= g) lp_at(S, c0n + 8 + g, c0n + 8 + j) = l2;
 		}
 	}
 	__syncwarp();
-	if (lane < CHOL_NB) Lt[lane * 17 + 16] = (lane < nbk) ? (T)dinv[c0 + lane] : T(1);
-	__syncwarp();
-}
-
-// Warp 0: factor the diagonal block at column c0 (nbk <= 16 real columns; the
-// padding is the identity) in FP64 registers; write L_KK back into S, 1/L_jj
-// into dinv[c0+j] (FP64), the first bad pivot (j+1) into *bad, and for the
-// panel solve a row-major 16x17 copy Lt of L_KK in the working precision with
-// the reciprocal pivots in column 16.
-template <typename T, bool REP = false>
-__device__ void chol_diag_factor(T *S, int c0, int nbk, double *dinv, T *Lt, int *bad) {
-	const int lane = threadIdx.x & 31;
-	T r[CHOL_NB];
-#pragma unroll
-	for (int l = 0; l < CHOL_NB; l++) {
-		T x = T(0);
-		if (lane < CHOL_NB && l <= lane) {
-			if (lane < nbk && l < nbk)
-				x = lp_at(S, c0 + lane, c0 + l);
-			else if (l == lane)
-				x = T(1);
-		}
-		r[l] = x;
-	}
-	if constexpr (REP && sizeof(T) == 4) {
-		if (lane < CHOL_NB) {
-#pragma unroll
-			for (int l = 0; l < CHOL_NB; l++) Lt[lane * 17 + l] = r[l];
-		}
-		__syncwarp();
-		diag_factor_rep<T>(Lt, nbk, c0, dinv, bad, r, lane);
-		__syncwarp();  // every lane has read the staged block before it is overwritten
-	} else {
-		DiagCol<0, T>::run(r, lane, nbk, c0, dinv, bad);
-	}
-	chol_diag_store<T>(S, c0, nbk, dinv, Lt, r, lane);
-}
-
-// Warp 0, look-ahead step: the rank-16 update of diagonal block K+1 (columns
-// c0n..c0n+15) with the panel of block column K (columns c0..c0+15, already
-// solved), fused with its factorization.  Lane i (and lane i+16) own row i of
-// the block; the two half-warps take 8 of the 16 panel columns each, reading
-// the panel rows of the block as broadcast tile-column loads, and their
-// partial sums meet by one shuffle.  The update runs in the working precision
-// T, the factorization in FP64 registers (DiagCol).  Outputs as
-// chol_diag_factor.
-template <typename T, bool REP = false>
-__device__ void chol_diag_update_factor(T *S, int c0n, int nbk, int c0, double *dinv, T *Lt, int *bad) {
-	const int lane = threadIdx.x & 31;
-	const int i = lane & 15, h = lane >> 4;
-	const int pn = c0n >> 2, kb = c0 >> 2;
-	T u[CHOL_NB];
-#pragma unroll
-	for (int l = 0; l < CHOL_NB; l++) u[l] = (h == 0 && l <= i && i < nbk && l < nbk) ? lp_at(S, c0n + i, c0n + l) : T(0);
-	// row i of the panel block, the half-warp's 8 columns
-	T pr[8];
-#pragma unroll
-	for (int l = 0; l < 8; l++) pr[l] = (i < nbk) ? lp_at(S, c0n + i, c0 + 8 * h + l) : T(0);
-#pragma unroll
-	for (int jq = 0; jq < 4; jq++) {
-		if (4 * jq >= nbk) break;  // row panels past the end of the matrix
-#pragma unroll
-		for (int l = 0; l < 8; l++) {
-			const int col = 8 * h + l;
-			T v0, v1, v2, v3;
-			tile_col_ld<T>(S, pn + jq, kb + (col >> 2), col & 3, v0, v1, v2, v3);
-			u[4 * jq] = fma(-pr[l], v0, u[4 * jq]);
-			u[4 * jq + 1] = fma(-pr[l], v1, u[4 * jq + 1]);
-			u[4 * jq + 2] = fma(-pr[l], v2, u[4 * jq + 2]);
-			u[4 * jq + 3] = fma(-pr[l], v3, u[4 * jq + 3]);
-		}
-	}
-	T r[CHOL_NB];
-#pragma unroll
-	for (int l = 0; l < CHOL_NB; l++) {
-		const T s = u[l] + __shfl_xor_sync(0xffffffffu, u[l], 16);
-		// real entries of the lower triangle; identity in the padding
-		r[l] = (l <= i && i < nbk && l < nbk) ? s : ((l == i && i >= nbk) ? T(1) : T(0));
-	}
-	if constexpr (REP && sizeof(T) == 4) {
-		if (lane < CHOL_NB) {
-#pragma unroll
-			for (int l = 0; l < CHOL_NB; l++) Lt[lane * 17 + l] = r[l];
-		}
-		__syncwarp();
-		diag_factor_rep<T>(Lt, nbk, c0n, dinv, bad, r, lane);
-		__syncwarp();  // every lane has read the staged block before it is overwritten
-	} else {
-		DiagCol<0, T>::run(r, lane, nbk, c0n, dinv, bad);
-	}
-	chol_diag_store<T>(S, c0n, nbk, dinv, Lt, r, lane);
 }
 
 // panel of block column c0, rows r in [rbeg, rend): substitution with the
@@ -447,20 +310,18 @@ __device__ __forceinline__ void chol_tile_update(T *S, int ti, int tj, int c0) {
 }
 
 // Full factorization of the n x n lower-panel matrix S by the whole CTA
-// (blockDim.x >= 64).  dinv: FP64 shared array of >= 4P entries; Lt: 16*17
-// entries of T; bad: shared int (0 on entry).  With inv_diag the diagonal
+// (blockDim.x >= 64).  dinv: FP64 shared array of >= 4P entries; Lt: CHOL_SCR
+// doubles (16-byte aligned), the row-major diagonal block first; bad: shared int (0 on entry).  With inv_diag the diagonal
 // blocks of the factor are replaced at the end by their explicit inverses
 // (all blocks in parallel), for the blocked triangular solves; the blocks
 // below the diagonal keep L.
-// REP (FP32 only, kernels with registers to spare): the diagonal blocks are
-// factored by diag_factor_rep instead of DiagCol.
-template <typename T, bool REP = false>
+template <typename T>
 __device__ void chol_smem(T *S, int n, double *dinv, T *Lt, int *bad, bool inv_diag) {
 	const int P = (n + 3) >> 2;
 	const int NB = (n + 15) >> 4;
 	const int tid = threadIdx.x, nt = blockDim.x;
 	const int warp = tid >> 5, lane = tid & 31;
-	if (warp == 0) chol_diag_factor<T, REP>(S, 0, min(CHOL_NB, n), dinv, Lt, bad);
+	if (warp == 0) chol_diag<T>(S, 0, min(CHOL_NB, n), -1, dinv, Lt, bad);
 	__syncthreads();
 	for (int K = 0; K < NB; K++) {
 		const int c0 = 16 * K, k0 = 4 * K;
@@ -472,7 +333,7 @@ __device__ void chol_smem(T *S, int n, double *dinv, T *Lt, int *bad, bool inv_d
 		// diagonal block K+1 belong to warp 0, which then factors that block
 		const int R = P - (k0 + 4);
 		if (warp == 0) {
-			chol_diag_update_factor<T, REP>(S, c0 + CHOL_NB, min(CHOL_NB, n - c0 - CHOL_NB), c0, dinv, Lt, bad);
+			chol_diag<T>(S, c0 + CHOL_NB, min(CHOL_NB, n - c0 - CHOL_NB), c0, dinv, Lt, bad);
 		} else if (warp & 3) {
 			// warps 4, 8, ... share warp 0's scheduler (warp w issues from
 			// sub-partition w % 4): they sit the update out so that the serial

@@ -10,8 +10,8 @@
 //            fragments are read from the factored columns in global memory --
 //            two 128-byte runs each in the panel layout, L2-resident while the
 //            CTA works on the matrix);
-//   factor:  warp 0 factors the 16 x 16 diagonal block in FP64 registers
-//            (DiagCol of chol.cuh: pivot rule of
+//   factor:  warp 0 factors the 16 x 16 diagonal block (frag::chol16, DiagCol
+//            for long matrices: pivot rule of
 //            kernel/generic/kernel_dgemm_4x4_lib4.c:5700-5710), the rows below
 //            solve their 16 entries against it (one thread per row,
 //            reciprocal-pivot multiply);
@@ -25,10 +25,13 @@
 
 constexpr int LL_PSTR = 17;  // shared-memory panel row stride (doubles)
 
+
+// doubles of the panel for an n x n matrix (the scratch behind it 16-byte aligned)
+__host__ __device__ inline size_t ll_panel(int n) { return ((size_t)(n + 8) * LL_PSTR + 1) & ~(size_t)1; }
 // shared memory of chol_ll for matrices up to max_n: the panel, the 16x17
-// diagonal factor with its reciprocal pivots
+// diagonal factor with its reciprocal pivots, the factorization's scratch
 __host__ __device__ inline size_t ll_smem_bytes(int max_n) {
-	return ((size_t)(max_n + 8) * LL_PSTR + 16 * 17) * sizeof(double);
+	return (ll_panel(max_n) + CHOL_SCR) * sizeof(double);
 }
 
 __device__ __forceinline__ void ll_dmma(double &d0, double &d1, double a, double b) {
@@ -44,13 +47,14 @@ __device__ __forceinline__ double ll_ld(const PMat<double> &d, int i, int k, int
 
 // Factor the n x n lower triangle of c into d (lower triangle of L, 1/L_jj in
 // d.d[j]); *bad (shared, zeroed by the caller) receives the first
-// non-positive pivot j+1.  All NT threads of the CTA call it.  FR: fragment
+// non-positive pivot j+1.  FRAG: diagonal blocks in tensor core fragments, else by
+// rows and shuffles.  All NT threads of the CTA call it.  FR: fragment
 // rows a warp updates at a time (its accumulators: 8 FR doubles per lane).
-template <int NT, int FR = 4>
+template <int NT, int FR = 4, bool FRAG = true>
 __device__ void chol_ll(const PMat<double> &c, const PMat<double> &d, int n, double *smem, int *bad) {
 	constexpr int NW = NT / 32;
 	double *pan = smem;
-	double *Lt = smem + (size_t)(n + 8) * LL_PSTR;
+	double *Lt = smem + ll_panel(n);
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int r = lane >> 2, q = lane & 3;
 	const int NBK = (n + 15) >> 4;
@@ -113,19 +117,47 @@ __device__ void chol_ll(const PMat<double> &c, const PMat<double> &d, int n, dou
 			}
 		}
 		__syncthreads();
-		// ---- diagonal block (warp 0, FP64 registers) ----
+		// ---- diagonal block (warp 0) ----
 		const int nbk = m < 16 ? m : 16;
 		if (warp == 0) {
-			double rv[CHOL_NB];
+			// padding rows of the panel hold the identity
+			double *scr = Lt + 16 * 17;
+			double v;
+			if constexpr (FRAG) {
+				double F[3][2];
 #pragma unroll
-			for (int l = 0; l < CHOL_NB; l++) rv[l] = (lane < CHOL_NB && l <= lane) ? pan[lane * LL_PSTR + l] : 0.0;
-			DiagCol<0, double>::run(rv, lane, nbk, c0, d.d, bad);
-			if (lane < CHOL_NB) {
+				for (int h = 0; h < 2; h++) {
+					const int j = 2 * q + h;
+					F[0][h] = j <= r ? -pan[r * LL_PSTR + j] : 0.0;
+					F[1][h] = 8 < m ? -pan[(8 + r) * LL_PSTR + j] : 0.0;
+					F[2][h] = j <= r ? (8 < m ? -pan[(8 + r) * LL_PSTR + 8 + j] : (j == r ? -1.0 : 0.0)) : 0.0;
+				}
+				v = frag::chol16(F, scr, lane);
+				const unsigned z = __ballot_sync(0xffffffffu, lane < nbk && frag::bad_pivot(v));
+				if (z && lane == 0 && *bad == 0) *bad = c0 + __ffs(z);
+				v = fabs(v);
 #pragma unroll
-				for (int l = 0; l < CHOL_NB; l++) Lt[lane * 17 + l] = (l <= lane) ? rv[l] : 0.0;
-				// the lane that computed pivot `lane` wrote d.d[c0 + lane]
-				Lt[lane * 17 + 16] = (lane < nbk) ? d.d[c0 + lane] : 1.0;
+				for (int h = 0; h < 2; h++) {
+					const int j = 2 * q + h;
+					Lt[r * 17 + j] = j <= r ? F[0][h] : 0.0;
+					Lt[r * 17 + 8 + j] = 0.0;
+					Lt[(8 + r) * 17 + j] = F[1][h];
+					Lt[(8 + r) * 17 + 8 + j] = j <= r ? F[2][h] : 0.0;
+				}
+			} else {
+				double rv[CHOL_NB];
+#pragma unroll
+				for (int l = 0; l < CHOL_NB; l++) rv[l] = (lane < CHOL_NB && l <= lane) ? pan[lane * LL_PSTR + l] : 0.0;
+				DiagCol<0, double>::run(rv, lane, nbk, c0, scr - c0, bad);
+				__syncwarp();
+				v = lane < nbk ? scr[lane] : 1.0;
+				if (lane < CHOL_NB) {
+#pragma unroll
+					for (int l = 0; l < CHOL_NB; l++) Lt[lane * 17 + l] = (l <= lane) ? rv[l] : 0.0;
+				}
 			}
+			if (lane < nbk) d.d[c0 + lane] = v;
+			if (lane < 16) Lt[lane * 17 + 16] = v;
 		}
 		__syncthreads();
 		// ---- rows below the diagonal block: x = a L_KK^{-T} ----

@@ -221,18 +221,14 @@ __device__ __forceinline__ void chol_pivot(double c, double &d, double &inv) {
 // from rsqrt over 1e8 values).  rsqrt() itself branches to its slow path for
 // subnormal and infinite arguments, and a branch per pivot keeps the compiler
 // from overlapping one column's update with the next column's pivot: this form
-// has 49 cycles of latency against 66 and no branch.  The caller collects
-// chol_odd and repeats the factorization with rsqrt() when any pivot was
-// outside the range.
+// has 49 cycles of latency against 66 and no branch.  A subnormal or infinite c
+// gives no finite number; the caller then repeats the factorization with
+// rsqrt().
 __device__ __forceinline__ double chol_rsqrt(double c) {
 	double y;
 	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(c));
 	const double e = fma(-(c * y), y, 1.0);
 	return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-// positive pivots that chol_rsqrt does not take: subnormal or infinite
-__device__ __forceinline__ bool chol_odd(double c) {
-	return (unsigned)(__double2hiint(c) - 0x00100000) >= 0x7fe00000u;
 }
 
 __host__ __device__ __forceinline__ int cdiv(int a, int b) { return (a + b - 1) / b; }

@@ -31,8 +31,8 @@ namespace {
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) / 16 * 16; }
 
 // shared-memory plan of the potrf kernel for matrices up to max_n
-// (lower panels, FP64 reciprocal pivots, the 16x17 row-major copy of the
-// diagonal block that chol_smem's panel solve reads, the bad-pivot flag)
+// (lower panels, FP64 reciprocal pivots, chol_smem's scratch with the 16x17
+// row-major copy of the diagonal block, the bad-pivot flag)
 struct PotrfSmem {
 	size_t s_bytes, dinv_off, lt_off, bad_off, total;
 };
@@ -43,7 +43,7 @@ __host__ __device__ inline PotrfSmem potrf_smem_plan(int max_n) {
 	p.s_bytes = align16((size_t)lp_size(max_n) * sizeof(T));
 	p.dinv_off = p.s_bytes;
 	p.lt_off = p.dinv_off + align16((size_t)4 * P * sizeof(double));
-	p.bad_off = p.lt_off + align16(16 * 17 * sizeof(T));
+	p.bad_off = p.lt_off + CHOL_SCR * sizeof(double);
 	p.total = p.bad_off + 16;
 	return p;
 }
@@ -1194,8 +1194,9 @@ int potrf_launch(int batch, SizeArg sz, int max_m, MatArg<T> C, MatArg<T> D, int
 			// L2 with FP64 tensor-core updates (at n = 128 0.11 ms against
 			// 0.15 ms for the shared-memory kernel); one launch per range, each
 			// kernel skips the instances of the other range
-			int st = dpotrf_dmma_launch(batch, sz, 64, C, D, info, s);
-			if (st || max_m <= 64) return st;
+			// (uniform sizes above 64 have nothing in the first)
+			const int st = sz.pm ? dpotrf_dmma_launch(batch, sz, 64, C, D, info, s) : BLASFEO_B200_OK;
+			if (st) return st;
 			return dpotrf_ll_launch(batch, sz, 64, max_m, C, D, info, s);
 		}
 	}

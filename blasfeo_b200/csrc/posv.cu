@@ -102,7 +102,7 @@ __host__ __device__ inline PosvPlan posv_plan(int max_n, int nt) {
 	const int P = (max_n + 3) / 4;
 	const int NB = (max_n + 15) / 16;
 	const int nv = NB * 16;
-	const size_t scr = (16 * 17 + 64) * sizeof(double);
+	const size_t scr = (CHOL_SCR + 32) * sizeof(double);
 	const size_t asum = MIXED ? (size_t)nv * sizeof(double) : 0;
 	p.S_off = 0;
 	p.dinv_off = p.S_off + a16((size_t)lp_size(max_n) * sizeof(T));

@@ -45,7 +45,7 @@ __host__ __device__ constexpr int lower_panels(int n8) { return 8 * (n8 / 4) * (
 __host__ __device__ constexpr int warp_doubles(int n8) { return lower_panels(8 * n8) + 80; }
 
 // The same factorization column by column in global memory by one warp, for
-// matrices with a pivot that chol_rsqrt does not take (subnormal or infinite)
+// matrices with a pivot that frag::panel does not take (subnormal, infinite, NaN)
 __device__ __noinline__ void potrf_warp(PMat<double> c, PMat<double> d, int n, int *info, int lane) {
 	int bad = 0;
 	for (int j = 0; j < n; j++)
@@ -79,7 +79,7 @@ __device__ __forceinline__ void factor(double (&F)[N8 * (N8 + 1) / 2][2], double
 			P[I - K][0] = F[blk(I, K)][0];
 			P[I - K][1] = F[blk(I, K)][1];
 		}
-		frag::panel<N8 - K, true>(P, sc, dv + 8 * K, r, q);
+		frag::panel<N8 - K>(P, sc, dv + 8 * K, r, q);
 		// trailing update, next panel's column first, the first step of every
 		// block of a column before the second
 #pragma unroll
@@ -154,20 +154,24 @@ __global__ void __launch_bounds__(32 * WPC, MINB) k_potrf_dmma(int batch, SizeAr
 	__syncwarp();
 	const double i0 = dv[lane], i1 = N8 > 4 ? dv[N8 > 4 ? 32 + lane : 0] : 1.0;
 	const double inf = __longlong_as_double(0x7ff0000000000000LL);
-	if (__any_sync(FULL, (lane < 8 * N8 && !(i0 < inf)) || (32 + lane < 8 * N8 && !(i1 < inf)))) {
+	bool odd = (lane < 8 * N8 && !(i0 < inf)) || (32 + lane < 8 * N8 && !(i1 < inf));
+#pragma unroll
+	for (int I = 0; I < N8; I++) odd |= frag::odd_diag(F[blk(I, I)], r, q);
+	if (__any_sync(FULL, odd)) {
 		potrf_warp(c, d, n, info ? info + b : nullptr, lane);
 		return;
 	}
-	if (lane < n) d.d[lane] = i0;
-	if (32 + lane < n) d.d[32 + lane] = i1;
-	const unsigned z0 = __ballot_sync(FULL, lane < n && i0 == 0.0), z1 = __ballot_sync(FULL, 32 + lane < n && i1 == 0.0);
+	if (lane < n) d.d[lane] = fabs(i0);
+	if (32 + lane < n) d.d[32 + lane] = fabs(i1);
+	const unsigned z0 = __ballot_sync(FULL, lane < n && frag::bad_pivot(i0)),
+	               z1 = __ballot_sync(FULL, 32 + lane < n && frag::bad_pivot(i1));
 	const int bad = z0 ? __ffs(z0) : (z1 ? 32 + __ffs(z1) : 0);
 	if (bad) {
 #pragma unroll
 		for (int I = 0; I < N8; I++)
 #pragma unroll
 			for (int h = 0; h < 2; h++)
-				if (r == 2 * q + h && dv[8 * I + r] == 0.0) F[blk(I, I)][h] = 0.0;
+				if (r == 2 * q + h && frag::bad_pivot(dv[8 * I + r])) F[blk(I, I)][h] = 0.0;
 	}
 
 	// store the lower triangle of L

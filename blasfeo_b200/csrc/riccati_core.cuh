@@ -34,8 +34,7 @@
 // lower L out: 0.073 ms there) are the floor.
 #pragma once
 
-#include <type_traits>
-
+#include "chol_frag.cuh"
 #include "quad.cuh"
 
 namespace ric {
@@ -68,11 +67,7 @@ __device__ __forceinline__ void cpa8(double *dst, const double *src) {
 	asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
 }
 
-__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
-	asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-	             : "+d"(d0), "+d"(d1)
-	             : "d"(a), "d"(b));
-}
+using frag::dmma;
 
 // stage k's inputs of the CTA's problems, interleaved slab: thread = (problem
 // t % 8, row t / 8 % 16, RSQ or BAbt), 8 bytes per copy; 8 problems of an
@@ -152,10 +147,11 @@ __device__ __forceinline__ void store_l(const Args &a, int k, int b0, const doub
 // the panel's diagonal block (finite values right of its diagonal), B (TWO)
 // the block below it, columns c0.. of L to Ls (row-major) with zeros above the
 // diagonal, inverse pivots to dv (0 for a pivot that is not positive), pv: 16
-// entries through which the pivots reach the warp.  keep: the lane's entries
+// entries through which the pivots reach the warp.  Valid while every number
+// is finite (frag::panel).  keep: the lane's entries
 // of B's factored columns 2q and 2q + 1, the operands of the next panel's
 // update.
-template <bool TWO, bool FAST>
+template <bool TWO>
 __device__ __forceinline__ void panel(double (&D)[2], double (&B)[2], double (&keep)[2], double *Ls, double *dv, double *pv,
                                       int c0, int g, int q) {
 	double *col = Ls + (c0 + g) * LD + c0 + 2 * q;
@@ -167,7 +163,7 @@ __device__ __forceinline__ void panel(double (&D)[2], double (&B)[2], double (&k
 		__syncwarp();
 		const double p = pv[c0 + c];
 		const bool ok = p > 0.0;
-		const double iv = FAST ? chol_rsqrt(p) : rsqrt(p);
+		const double iv = chol_rsqrt(p);
 		// the column's lanes scale it; zeros elsewhere (and above the diagonal)
 		// make it a rank-1 operand
 		const double l0 = D[e] * (ok && mine && g >= c ? iv : 0.0);
@@ -279,23 +275,32 @@ __global__ void __launch_bounds__(NT, 4) k_ric_trf_dmma(Args a) {
 		}
 		sync();  // every read of stage k's inputs and of L_{k+1} is done
 		if (k > 0) load(k - 1);
-		auto factor = [&](auto fast) {
-			constexpr bool FAST = decltype(fast)::value;
-			double A0[2] = {F0[0], F0[1]}, A1[2] = {F1[0], F1[1]}, A2[2] = {F2[0], F2[1]}, keep[2] = {0.0, 0.0};
-			panel<true, FAST>(A0, A1, keep, Ls, dv, pv, 0, g, q);
-			dmma(A2[0], A2[1], -keep[0], keep[0]);
-			dmma(A2[0], A2[1], -keep[1], keep[1]);
-			panel<false, FAST>(A2, A1, keep, Ls, dv, pv, 8, g, q);
+		double A0[2] = {F0[0], F0[1]}, A1[2] = {F1[0], F1[1]}, A2[2] = {F2[0], F2[1]}, keep[2] = {0.0, 0.0};
+		panel<true>(A0, A1, keep, Ls, dv, pv, 0, g, q);
+		dmma(A2[0], A2[1], -keep[0], keep[0]);
+		dmma(A2[0], A2[1], -keep[1], keep[1]);
+		panel<false>(A2, A1, keep, Ls, dv, pv, 8, g, q);
+		__syncwarp();
+		double iv = dv[lane & 15];
+		bool odd = !(iv < __longlong_as_double(0x7ff0000000000000LL)) || !(Ls[(lane & 15) * (LD + 1)] >= 0.0);
+		if (__any_sync(0xffffffffu, odd)) {
+			// a pivot that panel() does not take: by rows (chol_frag.cuh)
+			double G[3][2] = {{-F0[0], -F0[1]}, {-F1[0], -F1[1]}, {-F2[0], -F2[1]}};
 			__syncwarp();
-			return dv[lane & 15];
-		};
-		double iv = factor(std::true_type());
-		// chol_rsqrt returns no finite number for a pivot outside its range
-		if (__any_sync(0xffffffffu, !(iv < __longlong_as_double(0x7ff0000000000000LL)))) iv = factor(std::false_type());
-		const unsigned zero = __ballot_sync(0xffffffffu, lane < m && iv == 0.0);
-		if (zero) {
-			if (lane < m && iv == 0.0) Ls[lane * LD + lane] = 0.0;
-			if (first == 0) first = (N - k) * 16 + __ffs(zero);
+			frag::chol16_rows(G, dv - 16, lane);
+			*(double2 *)(Ls + g * LD + 2 * q) = make_double2(G[0][0], G[0][1]);
+			*(double2 *)(Ls + (8 + g) * LD + 2 * q) = make_double2(G[1][0], G[1][1]);
+			*(double2 *)(Ls + (8 + g) * LD + 8 + 2 * q) = make_double2(G[2][0], G[2][1]);
+			iv = dv[lane & 15];
+		}
+		const unsigned bad = __ballot_sync(0xffffffffu, lane < m && iv == 0.0);
+		if (bad) {
+			// L_jj and 1 / L_jj of a pivot that is not positive: 0
+			if (lane < m && iv == 0.0) {
+				if (!odd) Ls[lane * LD + lane] = 0.0;
+				dv[lane] = 0.0;
+			}
+			if (first == 0) first = (N - k) * 16 + __ffs(bad);
 			__syncwarp();
 		}
 	}
