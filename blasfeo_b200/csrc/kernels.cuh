@@ -14,9 +14,13 @@ template <bool LOWER>
 int dgemm_nt_dmma_launch(int batch, SizeArg sz, int max_m, int max_n, double alpha, MatArg<double> A,
                          MatArg<double> B, double beta, MatArg<double> C, MatArg<double> D, cudaStream_t s, int tile);
 
-// FP64 potrf_l for max_m <= 64, one warp per instance on the FP64 tensor cores (potrf_dmma.cu)
-int dpotrf_dmma_launch(int batch, SizeArg sz, int max_m, MatArg<double> C, MatArg<double> D, int *info,
-                       cudaStream_t s);
+// potrf_l and syrk_potrf_ln (D = chol(C + A B^T)) for max_m <= 64, one warp per
+// instance on the FP64 tensor cores (potrf_dmma.cu)
+template <typename T>
+int potrf_dmma_launch(int batch, SizeArg sz, int max_m, MatArg<T> C, MatArg<T> D, int *info, cudaStream_t s);
+template <typename T>
+int syrk_potrf_dmma_launch(int batch, SizeArg sz, int max_m, MatArg<T> A, MatArg<T> B, MatArg<T> C, MatArg<T> D,
+                           int *info, cudaStream_t s);
 
 // FP64 potrf_l for min_n < n <= max_m beyond shared memory: one CTA per
 // instance, left-looking panels with FP64 tensor-core updates (potrf_ll.cu)

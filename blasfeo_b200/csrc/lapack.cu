@@ -1186,8 +1186,8 @@ namespace bf {
 template <typename T>
 int potrf_launch(int batch, SizeArg sz, int max_m, MatArg<T> C, MatArg<T> D, int *info, cudaStream_t s, int variant) {
 	if (batch <= 0 || max_m <= 0) return BLASFEO_B200_OK;
+	if (max_m <= 64 && (variant < 0 || variant == 5)) return potrf_dmma_launch<T>(batch, sz, max_m, C, D, info, s);
 	if constexpr (sizeof(T) == 8) {
-		if (max_m <= 64 && (variant < 0 || variant == 5)) return dpotrf_dmma_launch(batch, sz, max_m, C, D, info, s);
 		if (variant < 0 && max_m <= dpotrf_ll_max_n()) {
 			// by size (measured fastest per range, uniform batches n = 32..384):
 			// n <= 64 one warp on the FP64 tensor cores, larger n blocked from
@@ -1195,7 +1195,7 @@ int potrf_launch(int batch, SizeArg sz, int max_m, MatArg<T> C, MatArg<T> D, int
 			// 0.15 ms for the shared-memory kernel); one launch per range, each
 			// kernel skips the instances of the other range
 			// (uniform sizes above 64 have nothing in the first)
-			const int st = sz.pm ? dpotrf_dmma_launch(batch, sz, 64, C, D, info, s) : BLASFEO_B200_OK;
+			const int st = sz.pm ? potrf_dmma_launch<T>(batch, sz, 64, C, D, info, s) : BLASFEO_B200_OK;
 			if (st) return st;
 			return dpotrf_ll_launch(batch, sz, 64, max_m, C, D, info, s);
 		}
@@ -1257,6 +1257,13 @@ void syrk_potrf_single(int m, int k, S *sA, int ai, int aj, S *sB, int bi, int b
 	if (m <= 0) return;
 	cudaStream_t s = bf::cur_stream();
 	MatArg<T> D = single_arg<T>(sD, di, dj);
+	if (m <= 64) {
+		sD->use_dA = (di == 0 && dj == 0) ? m : 0;
+		bf::syrk_potrf_dmma_launch<T>(1, uniform_sizes(m, m, k), m, single_arg<T>(sA, ai, aj), single_arg<T>(sB, bi, bj),
+		                              single_arg<T>(sC, ci, cj), D, nullptr, s);
+		bf::finish_single();
+		return;
+	}
 	bf::gemm_nt_launch<T, true>(1, uniform_sizes(m, m, k), m, m, k, T(1), single_arg<T>(sA, ai, aj),
 	                            single_arg<T>(sB, bi, bj), T(1), single_arg<T>(sC, ci, cj), D, s, -1);
 	sD->use_dA = (di == 0 && dj == 0) ? m : 0;
@@ -1271,6 +1278,12 @@ int syrk_potrf_batch(int batch, int m, int k, BT *sA, int ai, int aj, BT *sB, in
 	if (m <= 0 || batch == 0) return BLASFEO_B200_OK;
 	cudaStream_t s = (cudaStream_t)stream;
 	MatArg<T> D = batch_arg<T>(sD, di, dj);
+	if (m <= 64) {
+		// one kernel: the sum stays in the factorization's registers
+		sD->use_dA = (di == 0 && dj == 0) ? m : 0;
+		return bf::syrk_potrf_dmma_launch<T>(batch, uniform_sizes(m, m, k), m, batch_arg<T>(sA, ai, aj),
+		                                     batch_arg<T>(sB, bi, bj), batch_arg<T>(sC, ci, cj), D, info, s);
+	}
 	int st = bf::gemm_nt_launch<T, true>(batch, uniform_sizes(m, m, k), m, m, k, T(1), batch_arg<T>(sA, ai, aj),
 	                                     batch_arg<T>(sB, bi, bj), T(1), batch_arg<T>(sC, ci, cj), D, s, -1);
 	if (st) return st;
