@@ -153,75 +153,123 @@ __global__ void k_invdiag(SizeArg sz, MatArg<T> A) {
 // Element (i,k) is d_ik = (alpha b_ik - sum_{l<k} d_il a_kl) * inv_k with the
 // sum accumulated in increasing l.
 //
-// For n <= NMAX (16, 32, 64): the lower triangle of A and its
-// inverse diagonal are staged in shared memory once per CTA, and each row of
-// the right-hand side lives in registers, updated right-looking (after d_ij:
-// c_ik -= d_ij a_kj for k > j, A's column j read by every thread at once).
-// TPR threads share a row (columns interleaved, k = TPR q + h), so a row of 64
-// doubles fits in registers; the thread that owns column j passes d_ij to its
-// partner by a shuffle within the pair.  Element (i,k) sees alpha b_ik, then
-// the FMAs over l = 0..k-1 in order; nothing is re-read from global memory
-// inside the recurrence.  64 rows per CTA, blockDim.x = 64 TPR.
-template <typename T, bool UNIT, int NMAX, int TPR>
-__global__ void __launch_bounds__(64 * TPR) k_trsm_rltn_reg(SizeArg sz, T alpha, MatArg<T> A, MatArg<T> B,
-                                                             MatArg<T> D) {
-	constexpr int NQ = NMAX / TPR;
-	__shared__ T sa[NMAX * NMAX];  // sa[j * NMAX + k] = a(k, j), k > j
-	__shared__ T sinv[NMAX];
-	const int b = blockIdx.x;
-	const int m = sz.M(b), n = sz.N(b);
-	const PMat<T> a = A.get(b), bb = B.get(b), d = D.get(b);
-	{
-		// thread t stages row t % 64 of the columns j = t / 64 (mod TPR); the
-		// loop is unrolled so every load is in flight at once
-		const int k = threadIdx.x & 63, j0 = threadIdx.x >> 6;
+// R rows of the right-hand side per CTA, a thread each, in column blocks of 16:
+// block c0 starts as alpha b, receives the solved columns l < c0 (kept in
+// shared memory, xs[l R + row]) and is solved against its 16 x 16 diagonal
+// block, all in registers.  A's rows of every block are staged once, transposed
+// (as[.. + 16 l + k] = a(c0 + k, l)), so a step reads one column of 16 as
+// broadcast 16-byte loads for 16 FMAs.  The loops over blocks and solved columns
+// are rolled: the form with the whole row in registers (64 columns unrolled,
+// about 8,000 instructions run once per row) was bound by instruction fetch:
+// FP32, m = 60, n = 50 x 6,000 504 us, this kernel 129.  Shared memory:
+// A's blocks (8 nb (nb + 1) 16 entries), R columns of 16 nb, the inverse diagonal.
+__host__ __device__ inline size_t trsm_rows_elems(int n, int R) {
+	const int nb = (n + 15) >> 4;
+	return (size_t)128 * nb * (nb + 1) + (size_t)R * 16 * nb + 16 * nb;
+}
+
+template <typename T>
+__device__ __forceinline__ void ld16(T (&v)[16], const T *p) {
+	constexpr int E = 16 / sizeof(T);
 #pragma unroll
-		for (int jj = 0; jj < NQ; jj++) {
-			const int j = jj * TPR + j0;
-			if (j < n && k < n && k > j) sa[j * NMAX + k] = a.at(k, j);
+	for (int e = 0; e < 16; e += E) {
+		if constexpr (E == 4) {
+			const float4 x = *(const float4 *)(p + e);
+			v[e] = x.x;
+			v[e + 1] = x.y;
+			v[e + 2] = x.z;
+			v[e + 3] = x.w;
+		} else {
+			const double2 x = *(const double2 *)(p + e);
+			v[e] = x.x;
+			v[e + 1] = x.y;
 		}
-		if (!UNIT && threadIdx.x < n) sinv[threadIdx.x] = a.d[threadIdx.x];
-	}
-	__syncthreads();
-	const int h = threadIdx.x % TPR;
-	const int i = blockIdx.y * 64 + threadIdx.x / TPR;
-	if (i >= m) return;  // both threads of a pair leave together
-	const int lane = threadIdx.x & 31;
-	const unsigned pair = (TPR == 1) ? (1u << lane) : (3u << (lane & ~1));
-	T c[NQ];
-#pragma unroll
-	for (int q = 0; q < NQ; q++) {
-		const int k = q * TPR + h;
-		c[q] = (k < n) ? alpha * bb.at(i, k) : T(0);
-	}
-#pragma unroll
-	for (int j = 0; j < NMAX; j++) {
-		if (j >= n) break;
-		const int qj = j / TPR, hj = j % TPR;
-		T dj = T(0);
-		if (h == hj) dj = UNIT ? c[qj] : c[qj] * sinv[j];
-		if (TPR > 1) dj = __shfl_sync(pair, dj, (lane & ~(TPR - 1)) | hj);
-		if (h == hj) c[qj] = dj;
-#pragma unroll
-		for (int q = 0; q < NQ; q++) {
-			const int k = q * TPR + h;
-			if (k > j && k < n) c[q] = fma(-dj, sa[j * NMAX + k], c[q]);
-		}
-	}
-#pragma unroll
-	for (int q = 0; q < NQ; q++) {
-		const int k = q * TPR + h;
-		if (k < n) d.at(i, k) = c[q];
 	}
 }
 
-// n > 64: the same register solve by column blocks of 64.  Block J
+template <typename T, bool UNIT, int R, int NT>
+__global__ void __launch_bounds__(NT) k_trsm_rltn_rows(SizeArg sz, T alpha, MatArg<T> A, MatArg<T> B, MatArg<T> D) {
+	extern __shared__ __align__(16) unsigned char tr_smem[];
+	const int b = blockIdx.x;
+	const int m = sz.M(b), n = sz.N(b);
+	const PMat<T> a = A.get(b), bb = B.get(b), d = D.get(b);
+	const int nb = (n + 15) >> 4;
+	T *as = (T *)tr_smem, *xs = as + (size_t)128 * nb * (nb + 1), *sinv = xs + (size_t)R * 16 * nb;
+	const int tid = threadIdx.x;  // threads beyond the R rows only stage
+	// block K's 16 rows: columns 0 .. 16 K + 15 at as + 128 K (K + 1)
+	const bool vec = (a.ri & 3) == 0 && ((uintptr_t)a.p & 15) == 0;
+	for (int K = 0; K < nb; K++) {
+		T *dst = as + (size_t)128 * K * (K + 1);
+		const int nc = min(16 * K + 16, n);
+		if (vec) {
+			// four rows of a column at a time: one aligned run of the panel layout
+			for (int e = tid; e < 4 * nc; e += NT) {
+				const int p = e / nc, l = e - p * nc;
+				const int k = 16 * K + 4 * p;
+				if (k < n) {
+					const T *g = a.addr(k, l);
+					T *o = dst + 16 * l + 4 * p;
+					if constexpr (sizeof(T) == 4) {
+						*(float4 *)o = *(const float4 *)g;
+					} else {
+						*(double2 *)o = *(const double2 *)g;
+						*(double2 *)(o + 2) = *(const double2 *)(g + 2);
+					}
+				}
+			}
+		} else {
+			for (int e = tid; e < 16 * nc; e += NT) {
+				const int k = 16 * K + (e & 15), l = e >> 4;
+				if (k < n && k >= l) dst[e] = a.at(k, l);
+			}
+		}
+	}
+	if (!UNIT)
+		for (int l = tid; l < n; l += NT) sinv[l] = a.d[l];
+	__syncthreads();
+	const int i = blockIdx.y * R + tid;
+	if (tid >= R || i >= m) return;
+	T *x = xs + tid;
+	for (int K = 0; K < nb; K++) {
+		const int c0 = 16 * K, w = min(16, n - c0);
+		const T *ak = as + (size_t)128 * K * (K + 1);
+		T c[16], v[16];
+#pragma unroll
+		for (int k = 0; k < 16; k++) c[k] = k < w ? alpha * bb.at(i, c0 + k) : T(0);
+#pragma unroll 2
+		for (int l = 0; l < c0; l++) {
+			const T xl = -x[l * R];
+			ld16(v, ak + 16 * l);
+#pragma unroll
+			for (int k = 0; k < 16; k++) c[k] = fma(xl, v[k], c[k]);
+		}
+		// the diagonal block; columns >= w are not stored and reach no other
+#pragma unroll
+		for (int j = 0; j < 16; j++) {
+			if (j < w) {
+				if (!UNIT) c[j] *= sinv[c0 + j];
+				ld16(v, ak + 16 * (c0 + j));
+#pragma unroll
+				for (int k = j + 1; k < 16; k++) c[k] = fma(-c[j], v[k], c[k]);
+			}
+		}
+#pragma unroll
+		for (int k = 0; k < 16; k++)
+			if (k < w) {
+				d.at(i, c0 + k) = c[k];
+				x[(c0 + k) * R] = c[k];
+			}
+	}
+}
+
+// Beyond shared memory for k_trsm_rltn_rows: a row of 64 columns in registers
+// at a time, TPR threads share a row (columns interleaved, k = TPR q + h; the
+// thread that owns column j passes d_ij to its partner by a shuffle).  Block J
 // (columns c0 = 64 J ..) first receives the contributions of the solved
 // columns l < c0, -sum_l d_il a_kl, from chunks of 64 columns of A staged in
 // shared memory (d_il re-read from D, where the row's threads wrote it), then
-// runs the in-block recurrence of k_trsm_rltn_reg.  Element (i,k) again sees
-// alpha b_ik followed by the FMAs over l = 0..k-1 in increasing l, as in
-// k_trsm_rltn_reg.  Dynamic shared memory: two 64 x 64 blocks of
+// runs the in-block recurrence.  Element (i,k) again sees alpha b_ik followed by
+// the FMAs over l = 0..k-1 in increasing l.  Dynamic shared memory: two 64 x 64 blocks of
 // A and 64 inverse-diagonal entries.
 template <typename T, bool UNIT, int TPR>
 __global__ void __launch_bounds__(64 * TPR) k_trsm_rltn_blk(SizeArg sz, T alpha, MatArg<T> A, MatArg<T> B,
@@ -302,7 +350,7 @@ __global__ void __launch_bounds__(64 * TPR) k_trsm_rltn_blk(SizeArg sz, T alpha,
 // lane l holds the columns k = 2l, 2l + 1 of its row in registers; step j:
 // the owner lane finishes d_ij, a shuffle hands it to the warp, every lane
 // updates its columns k > j (same operations in the same order as
-// k_trsm_rltn_reg).  n <= 64.
+// k_trsm_rltn_rows).  n <= 64.
 template <typename T, bool UNIT>
 __global__ void __launch_bounds__(256) k_trsm_rltn_row(SizeArg sz, T alpha, MatArg<T> A, MatArg<T> B, MatArg<T> D) {
 	__shared__ T sa[64 * 64];  // sa[j * 64 + k] = a(k, j), k > j
@@ -352,13 +400,22 @@ void trsm_rltn_kernel(int batch, SizeArg sz, int m, int n, T alpha, MatArg<T> A,
 		k_trsm_rltn_row<T, UNIT><<<dim3(batch, cdiv(m, 8)), 256, 0, s>>>(sz, alpha, A, B, D);
 		return;
 	}
-	if (n <= 16)
-		k_trsm_rltn_reg<T, UNIT, 16, 1><<<grid, 64, 0, s>>>(sz, alpha, A, B, D);
-	else if (n <= 32)
-		k_trsm_rltn_reg<T, UNIT, 32, 1><<<grid, 64, 0, s>>>(sz, alpha, A, B, D);
-	else if (n <= 64)
-		k_trsm_rltn_reg<T, UNIT, 64, TPR64><<<grid, 64 * TPR64, 0, s>>>(sz, alpha, A, B, D);
-	else {
+	// A thread per row while at least two CTAs of 64 rows fit an SM, i.e. up to
+	// n = 152 in FP32 and n = 99 in FP64 (us, blocks of 64 columns / rows: FP32
+	// n = 96 x 2,000 472 / 264, n = 128 x 1,000 346 / 275, n = 192 x 500 449 /
+	// 1,047; FP64 n = 96 1,045 / 694, n = 128 645 / 1,046).  32 rows where there
+	// are no more, and for launches of a few matrices (while they fit at all):
+	// their rows then run on more SMs, with 256 threads to stage A (one matrix of
+	// n = 160: 128 / 61, FP32 145 / 57).
+	const bool few = (long long)batch * cdiv(m, 32) <= bf::num_sms();
+	const int R = (m <= 32 || few) ? 32 : 64;
+	const size_t rows_smem = trsm_rows_elems(n, R) * sizeof(T), most = few ? bf::max_smem_optin() : 100 * 1024;
+	if (rows_smem <= most) {
+		auto kern = few ? k_trsm_rltn_rows<T, UNIT, 32, 256>
+		                : (R == 32 ? k_trsm_rltn_rows<T, UNIT, 32, 32> : k_trsm_rltn_rows<T, UNIT, 64, 64>);
+		bf::smem_optin(kern, rows_smem);
+		kern<<<dim3(batch, cdiv(m, R)), few ? 256 : R, rows_smem, s>>>(sz, alpha, A, B, D);
+	} else {
 		const size_t smem = (2 * 64 * 64 + 64) * sizeof(T);
 		auto kern = k_trsm_rltn_blk<T, UNIT, TPR64>;
 		bf::smem_optin(kern, smem);
