@@ -35,6 +35,13 @@ bool dgetrf_reg_fits(int max_m, int max_n);
 int dgetrf_reg_launch(int batch, SizeArg sz, MatArg<double> C, MatArg<double> D, int *ipiv, long long stride, int *info,
                       cudaStream_t s, int max_m, int max_n, bool piv, int nt);
 
+// FP64 geqrf with the panels in registers (geqrf_reg.cu): whether it takes
+// matrices of up to max_m rows, and the launch with nt = 128, 256 or 512 threads
+// per matrix (raised where a matrix has more rows than fit)
+bool dgeqrf_reg_fits(int max_m);
+int dgeqrf_reg_launch(int batch, SizeArg sz, MatArg<double> C, MatArg<double> D, cudaStream_t s, int max_m, int max_n,
+                      int nt);
+
 // D = chol(C) lower, inverse diagonal into D's dA, info (device, may be null)
 template <typename T>
 int potrf_launch(int batch, SizeArg sz, int max_m, MatArg<T> C, MatArg<T> D, int *info, cudaStream_t s,

@@ -1293,7 +1293,8 @@ int syrk_potrf_batch(int batch, int m, int k, BT *sA, int ai, int aj, BT *sB, in
 
 // variant: -1 auto; 0..2: the blocked global-memory kernels (getrf FP64: register
 // panels with 128 / 256 / 512 threads, getrf_reg.cu; FP32: 128 threads with 4
-// or 2 blocks per SM, 256 threads; geqrf: 256 threads with the
+// or 2 blocks per SM, 256 threads; geqrf FP64: register panels with 128 / 256 /
+// 512 threads, geqrf_reg.cu; FP32: 256 threads with the
 // SIMT trailing update, 256 and 512 threads with the DMMA one); 3..5: the
 // instances whose block fits in shared memory there (128/256/512 threads),
 // the others in the blocked global-memory kernel (a second launch).
@@ -1353,8 +1354,7 @@ inline size_t lu_smem_bytes(int max_m, int max_n, size_t esz) {
 // batches timed on the B200 at n = 32..384: the shared-memory kernel with 128
 // threads for small blocks, the blocked global-memory kernels above (getrf, FP32:
 // 128 threads with 4 blocks per SM up to n = 96, with 2 up to 288, then 256
-// threads; geqrf: shared memory up to 64 rows, then the DMMA update with
-// 256 threads at 2 CTAs per SM)
+// threads; geqrf FP32: shared memory up to 64 rows, then 256 threads)
 inline int pick_lu_variant(int variant, int max_m, int max_n, bool qr = false) {
 	if (variant < 0) {
 		const int mx = max_m > max_n ? max_m : max_n;
@@ -1424,6 +1424,19 @@ int getrf_launch(int batch, SizeArg sz, MatArg<T> C, MatArg<T> D, int *ipiv, lon
 	return bf::check_launch();
 }
 
+// built-in rule for FP64 geqrf with register panels, by rows, from uniform batches
+// of 2n x n (ms; 128 / 256 / 512 threads): m = 64 x 20,000 1.35 / 2.41 / 4.65, m =
+// 128 x 20,000 5.29 / 6.41 / 11.2, m = 192 x 17,420 16.9 / 13.6 / 18.1, m = 256 x
+// 9,251 - / 13.0 / 15.1.  Launches of a few matrices take the next count: the
+// largest one sets the time (600 of up to 90 rows 79 / 58 us, 600 of up to 200
+// rows 256 / 512 threads 231 / 174).
+inline int pick_geqrf_reg(int batch, int max_m, bool uneven) {
+	const bool few = batch <= (uneven ? 6 : 2) * bf::num_sms();
+	if (max_m <= 64) return 0;
+	if (max_m <= 128) return few ? 1 : 0;
+	return max_m <= 256 && !few ? 1 : 2;
+}
+
 template <typename T>
 int geqrf_launch(int batch, SizeArg sz, MatArg<T> C, MatArg<T> D, cudaStream_t s, int max_m, int max_n,
                  int variant = -1) {
@@ -1431,6 +1444,13 @@ int geqrf_launch(int batch, SizeArg sz, MatArg<T> C, MatArg<T> D, cudaStream_t s
 	const size_t need = lu_smem_bytes(max_m, max_n, sizeof(T));
 	const size_t smem = need < cap_full ? need : cap_full;
 	const int cap = (int)smem;
+	if constexpr (sizeof(T) == 8) {
+		// up to 512 rows: the panel in registers, 128, 256 or 512 threads
+		if (variant < 3 && bf::dgeqrf_reg_fits(max_m)) {
+			if (variant < 0) variant = pick_geqrf_reg(batch, max_m, sz.pm != nullptr);
+			return bf::dgeqrf_reg_launch(batch, sz, C, D, s, max_m, max_n, 128 << variant);
+		}
+	}
 	variant = pick_lu_variant(variant, max_m, max_n, true);
 	switch (variant) {
 	// blocked: 256 threads with the SIMT update, 256 or 512 threads with the DMMA update

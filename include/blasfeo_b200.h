@@ -428,10 +428,10 @@ int blasfeo_dgeqrf_vbatch(int batch, const int *m, const int *n, int max_m, int 
  * op 2 getrf_rp: 0..2 blocked with the panel in registers, 128 (fewer for up to
  *   64 rows), 256 and 512 threads per matrix (more than 512 rows: blocked in
  *   global memory), 3..5 shared memory with 128/256/512 threads;
- * op 3 geqrf: 0..2 blocked in global memory (256 threads with the SIMT
- *   trailing update, 256 threads (2 per SM) and 512 threads with the FP64
- *   tensor-core update), 3..5
- *   shared memory with 128/256/512 threads.
+ * op 3 geqrf: 0..2 blocked with the panel in registers, 128 (64 for up to 32
+ *   rows), 256 and 512 threads per matrix (more threads where the rows need
+ *   them; more than 512 rows: blocked in global memory), 3..5 shared memory with
+ *   128/256/512 threads.
  * Variants change the schedule and, through the summation order of the dot
  * products, the rounding of an element; every variant meets the routine's
  * tolerance against the reference (pivot choices of getrf are identical). */
