@@ -314,9 +314,12 @@ __device__ __forceinline__ void chol_tile_update(T *S, int ti, int tj, int c0) {
 // doubles (16-byte aligned), the row-major diagonal block first; bad: shared int (0 on entry).  With inv_diag the diagonal
 // blocks of the factor are replaced at the end by their explicit inverses
 // (all blocks in parallel), for the blocked triangular solves; the blocks
-// below the diagonal keep L.
+// below the diagonal keep L.  w (optional, shared, 16 ceil(n/16) entries, zeros
+// from n on): overwritten by L^{-1} w, as one more row of each panel solve whose
+// update of the entries below runs beside the trailing update, so that the
+// forward substitution has no chain and no barriers of its own.
 template <typename T>
-__device__ void chol_smem(T *S, int n, double *dinv, T *Lt, int *bad, bool inv_diag) {
+__device__ void chol_smem(T *S, int n, double *dinv, T *Lt, int *bad, bool inv_diag, T *w = nullptr) {
 	const int P = (n + 3) >> 2;
 	const int NB = (n + 15) >> 4;
 	const int tid = threadIdx.x, nt = blockDim.x;
@@ -327,6 +330,18 @@ __device__ void chol_smem(T *S, int n, double *dinv, T *Lt, int *bad, bool inv_d
 		const int c0 = 16 * K, k0 = 4 * K;
 		// A. panel rows below the diagonal block
 		chol_panel_rows<T>(S, c0, c0 + CHOL_NB, 4 * P, tid, nt, Lt);
+		if (w && tid == nt - 1) {
+			T a[CHOL_NB];
+#pragma unroll
+			for (int c = 0; c < CHOL_NB; c++) {
+				T s = w[c0 + c];
+#pragma unroll
+				for (int l = 0; l < c; l++) s = fma(-a[l], Lt[c * 17 + l], s);
+				a[c] = s * Lt[c * 17 + 16];
+			}
+#pragma unroll
+			for (int c = 0; c < CHOL_NB; c++) w[c0 + c] = a[c];
+		}
 		__syncthreads();
 		if (K + 1 >= NB) break;
 		// B. trailing tiles (ti,tj), k0+4 <= tj <= ti < P; the 10 of the
@@ -349,6 +364,14 @@ __device__ void chol_smem(T *S, int n, double *dinv, T *Lt, int *bad, bool inv_d
 			// belong to warp 0.
 			const int nuw = (nt >> 5) - ((nt >> 5) + 3) / 4;
 			const int uw = warp - (warp >> 2) - 1;
+			if (w) {
+				for (int i = c0 + CHOL_NB + 32 * uw + lane; i < n; i += 32 * nuw) {
+					T s = w[i];
+#pragma unroll
+					for (int l = 0; l < CHOL_NB; l++) s = fma(-lp_at(S, i, c0 + l), w[c0 + l], s);
+					w[i] = s;
+				}
+			}
 			const int scmax = (R + 3) >> 2, sr = (R + 7) >> 3;
 			int si = 0, base = 0, cnt = scmax < 2 ? scmax : 2;
 			for (int sidx = uw;; sidx += nuw) {

@@ -7,8 +7,9 @@
 // class launched with the shared memory its largest member needs.
 //
 //   plain (T = double): lower triangle -> shared memory (lower panels, one HBM
-//     read), chol_smem, blocked forward/backward substitution (16x16 diagonal
-//     blocks by warp shuffles), x written once.  Matrices whose FP64 lower
+//     read), chol_smem, the forward substitution along with the
+//     factorization, blocked backward substitution (16x16 diagonal blocks by
+//     warp shuffles), x written once.  Matrices whose FP64 lower
 //     panels do not fit shared memory take the global-memory path
 //     (k_posv_global) instead.
 //   mixed (T = float): lower triangle converted to FP32 in shared memory,
@@ -118,39 +119,28 @@ __host__ __device__ inline PosvPlan posv_plan(int max_n, int nt) {
 }
 
 // Forward substitution w := L^{-1} w on the lower panels, 16-row blocks.
-// With inv_diag the diagonal blocks of S hold their inverses (chol_smem) and
-// the diagonal step is a 16x16 product; otherwise warp 0 substitutes with the
-// FP64 reciprocal pivots.
+// The diagonal blocks of S hold their inverses (chol_smem) and the diagonal step
+// is a 16x16 product.  (A system's first forward substitution goes along with
+// its factorization; these are the refinement's.)
 template <typename T>
-__device__ void trsv_fwd(const T *S, int n, bool inv_diag, const double *dinv, T *w, T *ybuf) {
+__device__ void trsv_fwd(const T *S, int n, T *w, T *ybuf) {
 	const int tid = threadIdx.x, nt = blockDim.x;
 	const int NB = (n + 15) >> 4;
 	for (int K = 0; K < NB; K++) {
 		const int c0 = 16 * K;
 		const int nbk = min(16, n - c0);
-		if (inv_diag) {
-			if (tid < 16) {
-				// all 16 entries of row tid of the block are read (the lower
-				// panels of a class hold 16 * NB rows and columns) and the ones
-				// outside the lower triangle masked by a select, so the loads
-				// need no branches
-				T s = T(0);
+		if (tid < 16) {
+			// all 16 entries of row tid of the block are read (the lower
+			// panels of a class hold 16 * NB rows and columns) and the ones
+			// outside the lower triangle masked by a select, so the loads
+			// need no branches
+			T s = T(0);
 #pragma unroll
-				for (int l = 0; l < 16; l++) {
-					const T v = lp_at(S, c0 + tid, c0 + l);
-					s = fma((l <= tid) ? v : T(0), w[c0 + l], s);
-				}
-				ybuf[tid] = (tid < nbk) ? s : T(0);
+			for (int l = 0; l < 16; l++) {
+				const T v = lp_at(S, c0 + tid, c0 + l);
+				s = fma((l <= tid) ? v : T(0), w[c0 + l], s);
 			}
-		} else if (tid < 32) {
-			const int lane = tid;
-			T v = (lane < nbk) ? w[c0 + lane] : T(0);
-			for (int k = 0; k < nbk; k++) {
-				T yk = __shfl_sync(0xffffffffu, v, k) * (T)dinv[c0 + k];
-				if (lane == k) v = yk;
-				if (lane > k && lane < nbk) v = fma(-lp_at(S, c0 + lane, c0 + k), yk, v);
-			}
-			if (lane < 16) ybuf[lane] = (lane < nbk) ? v : T(0);
+			ybuf[tid] = (tid < nbk) ? s : T(0);
 		}
 		__syncthreads();
 		// rows below the block, one 4-row panel per thread: each column of a
@@ -181,7 +171,9 @@ __device__ void trsv_fwd(const T *S, int n, bool inv_diag, const double *dinv, T
 	}
 }
 
-// Backward substitution w := L^{-T} w (inv_diag as trsv_fwd).
+// Backward substitution w := L^{-T} w.  With inv_diag the diagonal blocks of S
+// hold their inverses; otherwise warp 0 substitutes with the FP64 reciprocal
+// pivots, the block's column l in lane l's registers before the 16-step chain.
 template <typename T>
 __device__ void trsv_bwd(const T *S, int n, bool inv_diag, const double *dinv, T *w, T *ybuf) {
 	const int tid = threadIdx.x, nt = blockDim.x;
@@ -202,10 +194,16 @@ __device__ void trsv_bwd(const T *S, int n, bool inv_diag, const double *dinv, T
 		} else if (tid < 32) {
 			const int lane = tid;
 			T v = (lane < nbk) ? w[c0 + lane] : T(0);
-			for (int k = nbk - 1; k >= 0; k--) {
-				T xk = __shfl_sync(0xffffffffu, v, k) * (T)dinv[c0 + k];
-				if (lane == k) v = xk;
-				if (lane < k) v = fma(-lp_at(S, c0 + k, c0 + lane), xk, v);
+			const T rcp = (lane < nbk) ? (T)dinv[c0 + lane] : T(0);
+			T col[16];
+#pragma unroll
+			for (int k = 1; k < 16; k++) col[k] = (lane < k && k < nbk) ? lp_at(S, c0 + k, c0 + lane) : T(0);
+#pragma unroll
+			for (int k = 15; k >= 0; k--) {
+				const T x = v * rcp;
+				const T xk = __shfl_sync(0xffffffffu, x, k);
+				if (lane == k) v = x;
+				if (lane < k) v = fma(-col[k], xk, v);
 			}
 			if (lane < 16) ybuf[lane] = (lane < nbk) ? v : T(0);
 		}
@@ -461,14 +459,21 @@ __global__ void __launch_bounds__(NT, MINB) k_posv(int cls, int max_n, PosvWs ws
 			load_lp_vec<T, double, 4>(S, n, a.p, a.cn, MIXED ? slot : nullptr);
 		else
 			load_lp_vec<T, double, 2>(S, n, a.p, a.cn, MIXED ? slot : nullptr);
-		for (int i = tid; i < nv; i += nt) w[i] = (i < n) ? (T)bg[i] : T(0);
-		if (MIXED)
+		// the right-hand side (scaled to 1 for the FP32 solve) goes through the
+		// factorization, which does the first forward substitution
+		double scale = 1.0;
+		if (MIXED) {
+			double m = 0.0;
+			for (int i = tid; i < n; i += nt) m = fmax(m, fabs(bg[i]));
+			m = block_max<T>(m, misc);
+			scale = (m > 0.0) ? 1.0 / m : 1.0;
 			for (int i = tid; i < nv; i += nt) xs[i] = 0.0;
+		}
+		for (int i = tid; i < nv; i += nt) w[i] = (i < n) ? (T)(MIXED ? bg[i] * scale : bg[i]) : T(0);
 		__syncthreads();
-		chol_smem<T>(S, n, dinv, (T *)scratch, s_bad, MIXED);
+		chol_smem<T>(S, n, dinv, (T *)scratch, s_bad, MIXED, w);
 
 		if (!MIXED) {
-			trsv_fwd<T>(S, n, false, dinv, w, ybuf);
 			trsv_bwd<T>(S, n, false, dinv, w, ybuf);
 			for (int i = tid; i < n; i += nt) xg[i] = (double)w[i];
 			if (tid == 0) {
@@ -483,17 +488,8 @@ __global__ void __launch_bounds__(NT, MINB) k_posv(int cls, int max_n, PosvWs ws
 		double anorm = 0.0, bnorm_res = 0.0;
 		int it = 0;
 		bool conv = false;
-		double scale = 1.0;
-		{
-			double m = 0.0;
-			for (int i = tid; i < n; i += nt) m = fmax(m, fabs(bg[i]));
-			m = block_max<T>(m, misc);
-			scale = (m > 0.0) ? 1.0 / m : 1.0;
-			for (int i = tid; i < nv; i += nt) w[i] = (i < n) ? (T)(bg[i] * scale) : T(0);
-			__syncthreads();
-		}
 		for (;;) {
-			trsv_fwd<T>(S, n, true, dinv, w, ybuf);
+			if (it > 0) trsv_fwd<T>(S, n, w, ybuf);
 			trsv_bwd<T>(S, n, true, dinv, w, ybuf);
 			for (int i = tid; i < n; i += nt) xs[i] += (double)w[i] / scale;
 			__syncthreads();
@@ -554,20 +550,24 @@ __global__ void __launch_bounds__(NT, MINB) k_posv(int cls, int max_n, PosvWs ws
 	}
 }
 
-// Systems whose FP64 lower panels exceed shared memory: the factor goes to a
+// The larger systems of the plain solver: the factor goes to a
 // per-CTA workspace slot (panel layout, blocked left-looking with FP64
-// tensor-core updates, chol_ll.cuh), then the two blocked triangular solves
-// read it from there (L2-resident), the right-hand side in shared memory.
+// tensor-core updates, the forward substitution riding along, chol_ll.cuh), then
+// the backward substitution reads it from there (L2-resident), the right-hand
+// side in shared memory.
 __host__ __device__ inline size_t posv_slot_elems(int max_n) {
 	const size_t p4 = (size_t)(max_n + 3) / 4 * 4;
 	return p4 * p4 + (size_t)(max_n + 15) / 16 * 16;
 }
 constexpr int POSV_GLOBAL_NT = 128;
-// fragment rows per warp in the factorization's panel updates
-#ifndef POSV_GLOBAL_FR
-#define POSV_GLOBAL_FR 1
-#endif
-__global__ void __launch_bounds__(POSV_GLOBAL_NT, 4)
+constexpr int POSV_GLOBAL_MINB = 4;
+// Bound by the latency of L (L2) and of the diagonal blocks, so the registers
+// go to loads in flight: two fragment rows by four steps of 8 columns in the
+// panel update at 4 CTAs per SM (5,000 systems, n ~ U{4..256}: 1,102 us; one
+// fragment row 1,155, and at 5 / 6 CTAs with spills 1,332 / 1,370; eight steps
+// 1,197).  With the substitutions apart, L read step by step inside them, and
+// the other warps idle during the diagonal blocks: 1,635.
+__global__ void __launch_bounds__(POSV_GLOBAL_NT, POSV_GLOBAL_MINB)
     k_posv_global(int cls, int max_n, PosvWs ws, const int *__restrict__ nvec, const DevDesc<double> *__restrict__ sA,
                   const DevVec<double> *__restrict__ sb, const DevVec<double> *__restrict__ sx, double *slots,
                   int *info) {
@@ -603,8 +603,7 @@ __global__ void __launch_bounds__(POSV_GLOBAL_NT, 4)
 		a.ri = a.cj = 0;
 		const double *bg = sb[sys].pa;
 		for (int i = tid; i < n; i += POSV_GLOBAL_NT) y[i] = bg[i];
-		chol_ll<POSV_GLOBAL_NT, POSV_GLOBAL_FR>(a, L, n, pg_smem, &s_bad);
-		trsv_ll_fwd<POSV_GLOBAL_NT>(L, n, y);
+		chol_ll<POSV_GLOBAL_NT, 2, 4>(a, L, n, pg_smem, &s_bad, y);
 		trsv_ll_bwd<POSV_GLOBAL_NT>(L, n, y);
 		double *xg = sx[sys].pa;
 		for (int i = tid; i < n; i += POSV_GLOBAL_NT) xg[i] = y[i];
@@ -661,9 +660,13 @@ PosvLayout posv_layout(int batch, int max_n, bool use_slots) {
 	int smem_limit_n = 0;  // largest n the shared-memory kernel takes
 	for (int v = 4; v <= 4096; v += 4)
 		if (posv_plan<T, MIXED>(v, posv_threads(v)).total <= smem_cap) smem_limit_n = v;
-	// plain FP64: above n = 128 the blocked kernel with FP64 tensor-core
-	// updates (L2-resident factor, 4 systems per SM) beats the shared-memory one
-	if (!MIXED && smem_limit_n > 128) smem_limit_n = 128;
+	// plain FP64: the blocked kernel (L2-resident factor, FP64 tensor-core
+	// updates) from n = 65 on in calls that need its workspace anyway (5,000
+	// systems, n ~ U{4..256}: from 129 on 1,102 us, from 97 on 1,075, from 65 on
+	// 1,071); calls up to n = 128 keep to the shared-memory kernel, for which a
+	// workspace of blasfeo_dposv_worksize is enough
+	const int smem_max = max_n > 128 ? 64 : 128;
+	if (!MIXED && smem_limit_n > smem_max) smem_limit_n = smem_max;
 	for (int u : uppers) {
 		if (nc >= POSV_MAX_CLASSES - 1) break;
 		int uu = u < smem_limit_n ? u : smem_limit_n;
@@ -684,7 +687,7 @@ PosvLayout posv_layout(int batch, int max_n, bool use_slots) {
 	for (int c = 0; c < nc; c++) L.ct.upper[c] = L.cfg[c].upper;
 	// workspace: work list and class tables, global-path factor slots,
 	// mapped-path refinement slots
-	L.gslots = L.need_global ? 4 * bf::num_sms() : 0;
+	L.gslots = L.need_global ? POSV_GLOBAL_MINB * bf::num_sms() : 0;
 	L.need = posv_list_bytes((size_t)batch);
 	L.slots_off = L.need;
 	L.need += (size_t)L.gslots * posv_slot_elems(max_n) * sizeof(double);
