@@ -18,7 +18,6 @@
 //     the FP64 matrix in global memory (L2-resident while the CTA works on
 //     it), correction solves in FP32 with the stored block inverses, x += d in
 //     FP64, stopping when ||r||_inf <= tol * ||A||_inf * ||x||_inf.
-#include <climits>
 
 #include "chol.cuh"
 #include "chol_ll.cuh"
@@ -45,25 +44,34 @@ __global__ void k_posv_classify(int batch, const int *__restrict__ nvec, int max
 		atomicAdd(&hist[n], 1);
 	}
 	__syncthreads();
-	if (tid == 0) {
-		// descending n: bucket max_n+1 (oversize) first ... bucket 0 last
-		int acc = 0;
-		for (int v = max_n + 1; v >= 0; v--) {
-			off[v] = acc;
-			acc += hist[v];
+	if (tid < 32) {
+		// descending n: bucket max_n+1 (oversize) first ... bucket 0 last; a run of
+		// buckets per lane (the kernel took 17 us of a call at max_n = 256 with one
+		// thread over all of them; plain solver, 5,000 systems 1,072 -> 1,065 us, 300
+		// systems up to n = 100 111 -> 109)
+		const int run = (max_n + 2 + 31) / 32, top = max_n + 1 - tid * run;
+		int sum = 0;
+		for (int u = 0; u < run; u++)
+			if (top - u >= 0) sum += hist[top - u];
+		int acc = sum;
+#pragma unroll
+		for (int d = 1; d < 32; d <<= 1) {
+			const int o = __shfl_up_sync(0xffffffffu, acc, d);
+			if (tid >= d) acc += o;
 		}
-		for (int c = 0; c < ct.nclass; c++) {
-			int lo = (c == 0) ? 1 : ct.upper[c - 1] + 1;
-			int hi = ct.upper[c];
-			if (c == ct.nclass - 1) hi = max_n + 1;  // last class takes oversize too (kernel rejects)
-			int s = INT_MAX, cnt = 0;
-			for (int v = hi; v >= lo; v--) {
-				if (hist[v]) {
-					if (off[v] < s) s = off[v];
-					cnt += hist[v];
-				}
+		acc -= sum;
+		for (int u = 0; u < run; u++)
+			if (top - u >= 0) {
+				off[top - u] = acc;
+				acc += hist[top - u];
 			}
-			ws.start[c] = (cnt ? s : 0);
+		__syncwarp();
+		for (int c = tid; c < ct.nclass; c += 32) {
+			const int lo = (c == 0) ? 1 : ct.upper[c - 1] + 1;
+			// last class takes oversize too (kernel rejects)
+			const int hi = (c == ct.nclass - 1) ? max_n + 1 : ct.upper[c];
+			const int cnt = off[lo] + hist[lo] - off[hi];
+			ws.start[c] = cnt ? off[hi] : 0;
 			ws.count[c] = cnt;
 			ws.counter[c] = 0;
 		}
