@@ -217,7 +217,7 @@ int blasfeo_dsyrk_dpotrf_dtrsm_dgemm_batch(int batch, int m, int k, double shift
 	sD->use_dA = 0;
 	const ChainLayout lay = chain_layout(k);
 	const size_t smem = (size_t)lay.half_bytes * 2 * CH_WARPS;
-	cudaFuncSetAttribute(k_chain16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	bf::smem_optin(k_chain16, smem);
 	int per_sm = 0;
 	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_chain16, CH_WARPS * 32, smem);
 	if (per_sm < 1) per_sm = 1;

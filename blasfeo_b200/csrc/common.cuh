@@ -41,13 +41,16 @@ bool side_stream(cudaStream_t *stream, cudaEvent_t *fork, cudaEvent_t *join);
 // Let `kern` launch with `dyn` bytes of dynamic shared memory: the 48 KB that
 // a kernel gets without opting in cover its static and dynamic shared memory
 // together, so a launch whose dynamic part alone is below 48 KB can still
-// need the opt-in
+// need the opt-in.  The limit belongs to the kernel, not to the calling thread:
+// it is always set to the most the device gives, so that a thread with a small
+// launch does not lower it between another thread's opt-in and its launch.
 template <typename K>
 inline void smem_optin(K *kern, size_t dyn) {
 	cudaFuncAttributes a;
 	const size_t st = cudaFuncGetAttributes(&a, (const void *)kern) == cudaSuccess ? a.sharedSizeBytes : 0;
 	if (dyn + st > 48 * 1024)
-		cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+		cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                     (int)(max_smem_optin() - st));
 }
 
 template <typename T> struct MatT;

@@ -645,8 +645,7 @@ int launch_tc(int cls, int U, int batch, PosvWs ws, const int *n, const void *sA
 	const int max_ctas = (int)(512u / cols);
 	int per_sm = 0;
 	for (;;) {
-		if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-			return BLASFEO_B200_ECUDA;
+		bf::smem_optin(kern, smem);
 		if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem) != cudaSuccess)
 			return BLASFEO_B200_ECUDA;
 		if (per_sm <= max_ctas || smem >= cap) break;

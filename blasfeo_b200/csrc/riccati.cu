@@ -201,7 +201,7 @@ int ric_launch(int batch, int N, int nx, int nu, struct blasfeo_smat_batch *sBA,
 	if (info) cudaMemsetAsync(info, 0, sizeof(int) * batch, s);
 	const RicLayout<float> lay = ric_layout<float>(nx);
 	const size_t smem = (size_t)lay.warp_bytes * RIC_WARPS;
-	cudaFuncSetAttribute(k_ric_trf<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	bf::smem_optin(k_ric_trf<float>, smem);
 	int per_sm = 0;
 	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ric_trf<float>, RIC_WARPS * 32, smem);
 	if (per_sm < 1) per_sm = 1;
