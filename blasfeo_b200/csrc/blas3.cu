@@ -109,10 +109,9 @@ int gemm_nt_launch(int batch, SizeArg sz, int max_m, int max_n, int max_k, T alp
 		else
 			variant = mx > 48 ? 2 : (mx > 16 ? 1 : 0);
 	}
-	(void)max_k;
 	if constexpr (sizeof(T) == 8) {
 		if (variant == 4 || variant == 5)
-			return dgemm_nt_dmma_launch<LOWER>(batch, sz, max_m, max_n, alpha, A, B, beta, C, D, s, variant - 4);
+			return dgemm_nt_dmma_launch<LOWER>(batch, sz, max_m, max_n, max_k, alpha, A, B, beta, C, D, s, variant - 4);
 	}
 	switch (variant) {
 	case 0: return launch_gemm_cfg<T, 16, 16, 16, 2, 2, LOWER>(batch, sz, max_m, max_n, alpha, A, B, beta, C, D, s);

@@ -11,7 +11,7 @@ int gemm_nt_launch(int batch, SizeArg sz, int max_m, int max_n, int max_k, T alp
 
 // FP64 tensor-core (DMMA) gemm_nt / syrk_ln; tile 0 = 64x64, 1 = 32x32 (gemm_dmma.cu)
 template <bool LOWER>
-int dgemm_nt_dmma_launch(int batch, SizeArg sz, int max_m, int max_n, double alpha, MatArg<double> A,
+int dgemm_nt_dmma_launch(int batch, SizeArg sz, int max_m, int max_n, int max_k, double alpha, MatArg<double> A,
                          MatArg<double> B, double beta, MatArg<double> C, MatArg<double> D, cudaStream_t s, int tile);
 
 // potrf_l and syrk_potrf_ln (D = chol(C + A B^T)) for max_m <= 64, one warp per
