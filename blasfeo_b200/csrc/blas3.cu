@@ -400,20 +400,27 @@ void trsm_rltn_kernel(int batch, SizeArg sz, int m, int n, T alpha, MatArg<T> A,
 		return;
 	}
 	// A thread per row while at least two CTAs of 64 rows fit an SM, i.e. up to
-	// n = 152 in FP32 and n = 99 in FP64 (us, blocks of 64 columns / rows: FP32
+	// n = 160 in FP32 and n = 96 in FP64 (us, blocks of 64 columns / rows: FP32
 	// n = 96 x 2,000 472 / 264, n = 128 x 1,000 346 / 275, n = 192 x 500 449 /
 	// 1,047; FP64 n = 96 1,045 / 694, n = 128 645 / 1,046).  32 rows where there
-	// are no more, and for launches of a few matrices (while they fit at all):
-	// their rows then run on more SMs, with 256 threads to stage A (one matrix of
-	// n = 160: 128 / 61, FP32 145 / 57).
+	// are no more (up to n = 176 and 112), and for launches of a few matrices (while
+	// they fit at all): their rows then run on more SMs, with 256 threads to stage A
+	// (one matrix of n = 160: 128 / 61, FP32 145 / 57).  A thread per row to stage A
+	// up to n = 48, 128 beyond, where A is most of the work (thread per row / 128:
+	// FP32 n = 48, 32 rows x 2,000 20.4 / 24.3, n = 64 46.6 / 34.4, n = 176, 8 rows x
+	// 4,000 1,717 / 977 (blocks of 64 columns 985); 64 rows n = 152 x 2,000 550 / 486;
+	// FP64 n = 96, 100 rows x 2,000 697 / 645).
 	const bool few = (long long)batch * cdiv(m, 32) <= bf::num_sms();
 	const int R = (m <= 32 || few) ? 32 : 64;
 	const size_t rows_smem = trsm_rows_elems(n, R) * sizeof(T), most = few ? bf::max_smem_optin() : 100 * 1024;
 	if (rows_smem <= most) {
-		auto kern = few ? k_trsm_rltn_rows<T, UNIT, 32, 256>
-		                : (R == 32 ? k_trsm_rltn_rows<T, UNIT, 32, 32> : k_trsm_rltn_rows<T, UNIT, 64, 64>);
+		const int nt = few ? 256 : (n > 48 ? 128 : R);
+		auto kern = R == 64 ? (nt == 64 ? k_trsm_rltn_rows<T, UNIT, 64, 64> : k_trsm_rltn_rows<T, UNIT, 64, 128>)
+		            : nt == 256 ? k_trsm_rltn_rows<T, UNIT, 32, 256>
+		            : nt == 128 ? k_trsm_rltn_rows<T, UNIT, 32, 128>
+		                        : k_trsm_rltn_rows<T, UNIT, 32, 32>;
 		bf::smem_optin(kern, rows_smem);
-		kern<<<dim3(batch, cdiv(m, R)), few ? 256 : R, rows_smem, s>>>(sz, alpha, A, B, D);
+		kern<<<dim3(batch, cdiv(m, R)), nt, rows_smem, s>>>(sz, alpha, A, B, D);
 	} else {
 		const size_t smem = (2 * 64 * 64 + 64) * sizeof(T);
 		auto kern = k_trsm_rltn_blk<T, UNIT, TPR64>;
