@@ -28,13 +28,12 @@
 
 constexpr int LL_PSTR = 17;  // shared-memory panel row stride (doubles)
 
-// doubles of the panel for an n x n matrix (the scratch behind it 16-byte aligned)
+// doubles of the panel for an n x n matrix (what follows 16-byte aligned)
 __host__ __device__ inline size_t ll_panel(int n) { return ((size_t)(n + 8) * LL_PSTR + 1) & ~(size_t)1; }
-// shared memory of chol_ll for matrices up to max_n: the panel, the 16x17
-// diagonal factor with its reciprocal pivots, the factorization's scratch
-__host__ __device__ inline size_t ll_smem_bytes(int max_n) {
-	return (ll_panel(max_n) + CHOL_SCR) * sizeof(double);
-}
+// shared memory of chol_ll for matrices up to max_n: the panel, whose first 16 rows
+// are the diagonal factor with its reciprocal pivots in column 16, then 16x17
+// entries for the factorization's scratch
+__host__ __device__ inline size_t ll_smem_bytes(int max_n) { return (ll_panel(max_n) + 16 * 17) * sizeof(double); }
 
 __device__ __forceinline__ void ll_dmma(double &d0, double &d1, double a, double b) {
 	asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -81,7 +80,7 @@ __device__ void chol_ll(const PMat<double> &c, const PMat<double> &d, int n, dou
                         double *y = nullptr) {
 	__shared__ int next;  // fragment rows claimed in the panel at hand
 	double *pan = smem;
-	double *Lt = smem + ll_panel(n);
+	double *Lt = pan;  // row stride LL_PSTR = 17
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int r = lane >> 2, q = lane & 3;
 	const int NBK = (n + 15) >> 4;
@@ -98,7 +97,7 @@ __device__ void chol_ll(const PMat<double> &c, const PMat<double> &d, int n, dou
 		// ---- diagonal block: its update and factorization in warp 0's fragments,
 		// beside the other warps' updates of the rows below ----
 		if (warp == 0) {
-			double *scr = Lt + 16 * 17;
+			double *scr = pan + ll_panel(n);
 			double cv[3][2];
 #pragma unroll
 			for (int h = 0; h < 2; h++) {
@@ -201,7 +200,7 @@ __device__ void chol_ll(const PMat<double> &c, const PMat<double> &d, int n, dou
 			const int i = 4 * p + (w & 3), j = w >> 2;  // panel-relative row, column
 			const int gi = c0 + i, gj = c0 + j;
 			if (gi < n && gj < n && (i >= 16 || j <= i))
-				*d.addr(gi, gj) = (i < 16) ? Lt[i * 17 + j] : pan[i * LL_PSTR + j];
+				*d.addr(gi, gj) = pan[i * LL_PSTR + j];
 		}
 		__syncthreads();
 	}

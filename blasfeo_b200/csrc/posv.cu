@@ -710,6 +710,14 @@ PosvLayout posv_layout(int batch, int max_n, bool use_slots) {
 	return L;
 }
 
+// dynamic shared memory of k_posv_global: chol_ll's, then the right-hand side
+inline size_t posv_global_smem(int max_n) { return ll_smem_bytes(max_n) + (size_t)max_n * sizeof(double); }
+bool posv_global_fits(int max_n) {
+	cudaFuncAttributes a;
+	if (cudaFuncGetAttributes(&a, (const void *)k_posv_global) != cudaSuccess) return false;
+	return posv_global_smem(max_n) + a.sharedSizeBytes <= bf::max_smem_optin();
+}
+
 template <typename T, bool MIXED>
 int posv_run(int batch, const int *n, int max_n, const void *sA, const void *sb, const void *sx, int max_iter,
              double tol, int *iters, double *berr, int *info, void *work, size_t work_bytes, cudaStream_t s,
@@ -721,7 +729,8 @@ int posv_run(int batch, const int *n, int max_n, const void *sA, const void *sb,
 	const ClassTable ct = lay.ct;
 	const int nc = lay.nc;
 	const bool need_global = lay.need_global;
-	if (need_global && max_n > bf::dpotrf_ll_max_n()) return BLASFEO_B200_ENOTSUP;
+	// the panel and the right-hand side of the largest systems, before anything is launched
+	if (need_global && !posv_global_fits(max_n)) return BLASFEO_B200_ENOTSUP;
 	const int gslots = lay.gslots, rslots = lay.rslots;
 	const size_t need = lay.need, slots_off = lay.slots_off, rslots_off = lay.rslots_off;
 	char *wsp = (char *)work;
@@ -770,7 +779,7 @@ int posv_run(int batch, const int *n, int max_n, const void *sA, const void *sb,
 		const cudaStream_t s = (two && (ci & 1)) ? side : s0;
 		const bool glob = need_global && c == nc - 1;
 		if (glob) {
-			const size_t gsm = ll_smem_bytes(max_n) + (size_t)max_n * sizeof(double);
+			const size_t gsm = posv_global_smem(max_n);
 			bf::smem_optin(k_posv_global, gsm);
 			k_posv_global<<<gslots, POSV_GLOBAL_NT, gsm, s>>>(c, max_n, ws, n, (const DevDesc<double> *)sA,
 			                                                  (const DevVec<double> *)sb, (const DevVec<double> *)sx,
