@@ -1251,13 +1251,29 @@ int potrf_batch(int batch, int m, BT *sC, int ci, int cj, BT *sD, int di, int dj
 	                           info, (cudaStream_t)stream, -1);
 }
 
+// syrk_potrf_ln in one kernel (a warp forms the product and factors the sum), or
+// syrk_ln and potrf_l.  One kernel up to m = 64, but for launches of few matrices
+// with a long k: there the warp's own product takes longer than one spread over a
+// CTA or several.  us, two launches / one kernel: FP64 m = 64 x 1 k = 200 50 / 46, k =
+// 320 58 / 61, k = 1,000 112 / 148, x 200 k = 320 62 / 60, k = 1,000 129 / 147, x 300
+// k = 1,000 168 / 148; m = 48 x 1 k = 500 63 / 74; m = 40 x 1 k = 1,000 97 / 83; FP32
+// m = 48 x 32 k = 200 32 / 35, k = 1,000 94 / 114, x 100 106 / 113, m = 64 x 1 k = 1,000
+// 224 / 146, m = 40 90 / 91.
+template <typename T>
+bool syrk_potrf_fused(int batch, int m, int k) {
+	if (m > 64) return false;
+	const int sms = bf::num_sms();
+	if (sizeof(T) == 8) return !(m > 40 && 2LL * batch <= 3 * sms && k > (batch <= sms ? 256 : 400));
+	return !(m > 40 && m <= 48 && 2LL * batch <= sms && k > 200);
+}
+
 template <typename T, typename S>
 void syrk_potrf_single(int m, int k, S *sA, int ai, int aj, S *sB, int bi, int bj, S *sC, int ci, int cj, S *sD,
                        int di, int dj) {
 	if (m <= 0) return;
 	cudaStream_t s = bf::cur_stream();
 	MatArg<T> D = single_arg<T>(sD, di, dj);
-	if (m <= 64) {
+	if (syrk_potrf_fused<T>(1, m, k)) {
 		sD->use_dA = (di == 0 && dj == 0) ? m : 0;
 		bf::syrk_potrf_dmma_launch<T>(1, uniform_sizes(m, m, k), m, single_arg<T>(sA, ai, aj), single_arg<T>(sB, bi, bj),
 		                              single_arg<T>(sC, ci, cj), D, nullptr, s);
@@ -1278,7 +1294,7 @@ int syrk_potrf_batch(int batch, int m, int k, BT *sA, int ai, int aj, BT *sB, in
 	if (m <= 0 || batch == 0) return BLASFEO_B200_OK;
 	cudaStream_t s = (cudaStream_t)stream;
 	MatArg<T> D = batch_arg<T>(sD, di, dj);
-	if (m <= 64) {
+	if (syrk_potrf_fused<T>(batch, m, k)) {
 		// one kernel: the sum stays in the factorization's registers
 		sD->use_dA = (di == 0 && dj == 0) ? m : 0;
 		return bf::syrk_potrf_dmma_launch<T>(batch, uniform_sizes(m, m, k), m, batch_arg<T>(sA, ai, aj),
