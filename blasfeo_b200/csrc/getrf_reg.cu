@@ -82,10 +82,10 @@ __device__ __forceinline__ void warp_best(unsigned long long &key, int &pos, boo
 	pos = mp;
 }
 
-template <int NT, int RPT, int MINB>
+template <int NT, int RPT, int MINB, bool PIV>
 __global__ void __launch_bounds__(NT, MINB)
     k_getrf_reg(int batch, SizeArg sz, MatArg<double> C, MatArg<double> D, int *ipiv, long long ipiv_stride, int *info,
-                int max_m, int max_n, bool piv_on, int classes) {
+                int max_m, int max_n, int classes) {
 	constexpr int NW = NT / 32;
 	extern __shared__ __align__(16) unsigned char lu_sm[];
 	__shared__ unsigned long long s_key[2][NW];
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(NT, MINB)
 	short *rec = (short *)(lu_sm + pl.rec);            // per panel: count, then (row, from) pairs
 	const int ldu = pl.ch + 4;
 	const PMat<double> c = C.get(b), d = D.get(b);
-	int *piv = piv_on ? ipiv + ipiv_stride * b : nullptr;
+	int *piv = PIV ? ipiv + ipiv_stride * b : nullptr;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int g = lane >> 2, q = lane & 3;
 	for (int r = tid; r < m; r += NT) dmap[r] = -1;
@@ -133,49 +133,61 @@ __global__ void __launch_bounds__(NT, MINB)
 #pragma unroll
 		for (int j = 0; j < 16; j++) {
 			if (j < w) {
-				// the thread's candidate: among its rows at positions >= j (without
-				// pivoting only the row at position j)
-				unsigned long long key = 0;
-				int best = 0x7fffffff;
-				double row[16];
+				const double *ur;
+				int ip = j;
+				if (PIV) {
+					// the thread's candidate: among its rows at positions >= j
+					unsigned long long key = 0;
+					int best = 0x7fffffff;
+					double row[16];
 #pragma unroll
-				for (int l = j; l < 16; l++) row[l] = a[0][l];
+					for (int l = j; l < 16; l++) row[l] = a[0][l];
 #pragma unroll
-				for (int u = 0; u < RPT; u++) {
-					const bool act = pos[u] != 0x7fffffff && (piv_on ? pos[u] >= j : pos[u] == j);
-					const unsigned long long k = act ? lu_key(a[u][j]) : 0ULL;
-					if (act && (k > key || best == 0x7fffffff || (k == key && pos[u] < best))) {
-						key = k;
-						best = pos[u];
-						if (u > 0) {
+					for (int u = 0; u < RPT; u++) {
+						const bool act = pos[u] != 0x7fffffff && pos[u] >= j;
+						const unsigned long long k = act ? lu_key(a[u][j]) : 0ULL;
+						if (act && (k > key || best == 0x7fffffff || (k == key && pos[u] < best))) {
+							key = k;
+							best = pos[u];
+							if (u > 0) {
 #pragma unroll
-							for (int l = j; l < 16; l++) row[l] = a[u][l];
+								for (int l = j; l < 16; l++) row[l] = a[u][l];
+							}
 						}
 					}
-				}
-				bool win;
-				warp_best(key, best, win);
-				double *cr = crow + (size_t)((j & 1) * NW + warp) * 16;
-				if (win && best != 0x7fffffff) {
+					bool win;
+					warp_best(key, best, win);
+					double *cr = crow + (size_t)((j & 1) * NW + warp) * 16;
+					if (win && best != 0x7fffffff) {
 #pragma unroll
-					for (int l = j; l < 16; l++) cr[l] = row[l];
+						for (int l = j; l < 16; l++) cr[l] = row[l];
+					}
+					if (lane == 0) {
+						s_key[j & 1][warp] = key;
+						s_pos[j & 1][warp] = best;
+					}
+					__syncthreads();
+					key = lane < NW ? s_key[j & 1][lane] : 0ULL;
+					best = lane < NW ? s_pos[j & 1][lane] : 0x7fffffff;
+					warp_best(key, best, win);
+					ip = best;
+					ur = crow + (size_t)((j & 1) * NW + __ffs(__ballot_sync(FULL, win)) - 1) * 16;
+				} else {
+					// row j is thread j's first
+					double *cr = crow + (size_t)(j & 1) * NW * 16;
+					if (tid == j) {
+#pragma unroll
+						for (int l = j; l < 16; l++) cr[l] = a[0][l];
+					}
+					__syncthreads();
+					ur = cr;
 				}
-				if (lane == 0) {
-					s_key[j & 1][warp] = key;
-					s_pos[j & 1][warp] = best;
-				}
-				__syncthreads();
-				key = lane < NW ? s_key[j & 1][lane] : 0ULL;
-				best = lane < NW ? s_pos[j & 1][lane] : 0x7fffffff;
-				warp_best(key, best, win);
-				const int ip = best;
-				const double *ur = crow + (size_t)((j & 1) * NW + __ffs(__ballot_sync(FULL, win)) - 1) * 16;
 				const double pv = ur[j];
 				// getrf_rp: a zero pivot gives inverse 0; getrf_np divides as the
 				// reference does (blasfeo_ref/x_lapack_ref.c, REF_GETRF_NOPIVOT)
-				const double inv = piv_on ? (pv != 0.0 ? 1.0 / pv : 0.0) : 1.0 / pv;
+				const double inv = PIV ? (pv != 0.0 ? 1.0 / pv : 0.0) : 1.0 / pv;
 				if (tid == 0) {
-					if (piv_on) piv[c0 + j] = c0 + ip;
+					if (PIV) piv[c0 + j] = c0 + ip;
 					d.d[c0 + j] = inv;
 					if (pv == 0.0 && s_bad == 0) s_bad = c0 + j + 1;
 				}
@@ -310,7 +322,7 @@ __global__ void __launch_bounds__(NT, MINB)
 	// columns left of the panels: block K takes the row swaps of the panels
 	// after it, S[r] = the row whose content ends at r
 	const int np = (mn + 15) >> 4;
-	if (piv_on && np > 1) {
+	if (PIV && np > 1) {
 		for (int r = tid; r < m; r += NT) {
 			S[r] = (short)r;
 			dmap[r] = (short)r;
@@ -349,10 +361,10 @@ __global__ void __launch_bounds__(NT, MINB)
 template <int NT, int RPT, int MINB>
 int launch(int batch, SizeArg sz, MatArg<double> C, MatArg<double> D, int *ipiv, long long stride, int *info,
            cudaStream_t s, int max_m, int max_n, bool piv, int classes) {
-	auto kern = k_getrf_reg<NT, RPT, MINB>;
+	auto kern = piv ? k_getrf_reg<NT, RPT, MINB, true> : k_getrf_reg<NT, RPT, MINB, false>;
 	const size_t smem = lu_plan(NT, max_m, max_n).total;
 	bf::smem_optin(kern, smem);
-	kern<<<(unsigned)(batch * (long long)classes), NT, smem, s>>>(batch, sz, C, D, ipiv, stride, info, max_m, max_n, piv,
+	kern<<<(unsigned)(batch * (long long)classes), NT, smem, s>>>(batch, sz, C, D, ipiv, stride, info, max_m, max_n,
 	                                                              classes);
 	return bf::check_launch();
 }

@@ -1384,19 +1384,42 @@ inline int pick_lu_variant(int variant, int max_m, int max_n, bool qr = false) {
 	return variant;
 }
 
+// size by which FP64 getrf takes its threads: the larger one, but where the rows
+// are few the trailing columns are the work (us, no pivoting: 48 x 288 x 300 167 with
+// 512 threads, 105 with 256; 20 x 120 x 1 36 with 32, 23 with 64; 65 x 260 x 300 249 /
+// 166; pivoting and few matrices keep the threads for the search and the columns,
+// 100 x 200 x 1 125 with 512, 145 with 128)
+inline int getrf_reg_size(int batch, int max_m, int max_n, bool piv) {
+	if (max_m > 64 && (piv || max_m > 128 || batch <= bf::num_sms())) return max_m > max_n ? max_m : max_n;
+	return max_m > max_n / 2 ? max_m : max_n / 2;
+}
+
 // built-in rule for FP64 getrf with register panels, by matrix size, from
 // uniform batches (us; 128 / 256 / 512 threads): n = 128 x 9,251 3,654 / 4,428 /
 // 7,684, n = 160 x 5,662 4,706 / 4,000 / 6,494, n = 256 x 2,013 5,256 / 3,807 /
-// 5,169, n = 320 x 1,232 5,100 (256) / 5,322.  With one or two matrices per SM
-// the largest one sets the time and 512 threads finish it first (1,024 of sizes
-// log-uniform to 384: 1,136 / 741 for 256 / 512; 4,096: 3,621 / 3,961).
+// 5,169.  With few matrices per SM the largest one sets the time and 512 threads
+// finish it first (1,024 of sizes log-uniform to 384: 1,136 / 741 for 256 / 512;
+// 4,096: 3,621 / 3,961; uniform n = 320 x 1,232, 8 per SM, 5,100 / 5,322).
 // Uneven launches of a few hundred matrices are of that kind below n = 256 too
 // (600 of sizes to 200: 302 / 254).
-inline int pick_getrf_reg(int batch, int max_m, int max_n, bool uneven) {
-	const int mx = max_m > max_n ? max_m : max_n;
+inline int pick_getrf_reg(int batch, int max_m, int max_n, bool uneven, bool piv) {
+	const int mx = getrf_reg_size(batch, max_m, max_n, piv);
 	if (mx <= 128) return 0;
 	if (mx <= 256) return batch <= (uneven ? 6 : 2) * bf::num_sms() ? 2 : 1;
 	return batch <= 16 * bf::num_sms() ? 2 : 1;
+}
+
+// FP64 getrf of tiny and flat matrices, where the kernel with register panels has
+// too little to do for its set-up: variant of the others, or -1.  us, register
+// panels / here: no pivoting 3 x 4 x 148 8.3 / 4.3, 6 x 9 x 300 8.3 / 6.2, 48 x 2 x
+// 2,000 10.3 / 6.4 (unblocked in shared memory), 4 x 256 x 1 10.4 / 8.5 (blocked in
+// global memory; x 300 14.5 / 19.1); pivoting 3 x 6 x 300 8.3 / 6.3, 32 x 1 5.3 / 4.8.
+inline int pick_getrf_flat(int batch, int max_m, int max_n, bool piv) {
+	const int mx = max_m > max_n ? max_m : max_n, mn = max_m > max_n ? max_n : max_m, sms = bf::num_sms();
+	if (!piv && max_m <= 8 && max_n > 48 && max_n <= 256 && batch <= sms) return 2;
+	if (mx > 48 || (batch > 8 * sms && (piv || mn > 2))) return -1;
+	if (piv) return max_n == 1 || (max_m <= 3 && max_n >= 3 && max_n <= 8) ? 3 : -1;
+	return mn <= 4 || (mn <= 6 && mx <= 16) ? 3 : -1;
 }
 
 template <typename T>
@@ -1406,15 +1429,19 @@ int getrf_launch(int batch, SizeArg sz, MatArg<T> C, MatArg<T> D, int *ipiv, lon
 	const size_t need = lu_smem_bytes(max_m, max_n, sizeof(T));
 	const size_t smem = need < cap_full ? need : cap_full;
 	const int cap = (int)smem;
-	if (sizeof(T) == 8 && variant < 0 && bf::dgetrf_reg_fits(max_m, max_n))
-		variant = pick_getrf_reg(batch, max_m, max_n, sz.pm != nullptr);
+	const int flat = sizeof(T) == 8 && variant < 0 ? pick_getrf_flat(batch, max_m, max_n, piv) : -1;
+	if (flat >= 0)
+		variant = flat;
+	else if (sizeof(T) == 8 && variant < 0 && bf::dgetrf_reg_fits(max_m, max_n))
+		variant = pick_getrf_reg(batch, max_m, max_n, sz.pm != nullptr, piv);
 	variant = pick_lu_variant(variant, max_m, max_n);
 	if constexpr (sizeof(T) == 8) {
 		// up to 512 rows: the panel in registers, 128, 256 or 512 threads
 		// (variant 0: 32 or 64 where that covers the rows)
-		if (variant < 3 && bf::dgetrf_reg_fits(max_m, max_n))
+		const int size = getrf_reg_size(batch, max_m, max_n, piv);
+		if (variant < 3 && flat < 0 && bf::dgetrf_reg_fits(max_m, max_n))
 			return bf::dgetrf_reg_launch(batch, sz, C, D, ipiv, ipiv_stride, info, s, max_m, max_n, piv,
-			                             variant > 0 ? 128 << variant : (max_m <= 32 ? 32 : (max_m <= 64 ? 64 : 128)));
+			                             variant > 0 ? 128 << variant : (size <= 32 ? 32 : (size <= 64 ? 64 : 128)));
 	}
 	if constexpr (sizeof(T) == 8) {
 		// beyond the register panels: blocked in global memory
