@@ -293,14 +293,19 @@ __global__ void __launch_bounds__(NT, 4) k_ric_trf_dmma(Args a) {
 			*(double2 *)(Ls + (8 + g) * LD + 8 + 2 * q) = make_double2(G[2][0], G[2][1]);
 			iv = dv[lane & 15];
 		}
-		const unsigned bad = __ballot_sync(0xffffffffu, lane < m && iv == 0.0);
-		if (bad) {
-			// L_jj and 1 / L_jj of a pivot that is not positive: 0
-			if (lane < m && iv == 0.0) {
+		const bool zero = lane < m && iv == 0.0;
+		if (__any_sync(0xffffffffu, zero)) {
+			// L_jj and 1 / L_jj of a pivot that is not positive: 0.  An infinite
+			// pivot (1 / L_jj = 0, L_jj = inf * 0 = NaN) counts in info back to back,
+			// where it is L_jj that must be positive, but not interleaved, where it
+			// is the pivot (as in potrf_l on these slabs)
+			if (zero) {
 				if (!odd) Ls[lane * LD + lane] = 0.0;
 				dv[lane] = 0.0;
 			}
-			if (first == 0) first = (N - k) * 16 + __ffs(bad);
+			const bool inf = INTER && zero && Ls[lane * LD + lane] != 0.0;
+			const unsigned bad = __ballot_sync(0xffffffffu, zero && !inf);
+			if (bad && first == 0) first = (N - k) * 16 + __ffs(bad);
 			__syncwarp();
 		}
 	}
