@@ -72,7 +72,9 @@ __device__ __noinline__ void potrf_warp(PMat<T> c, PMat<T> d, PMat<T> a, PMat<T>
 		const double p = (double)d.at(j, j);
 		const bool ok = p > 0.0;
 		const double iv = ok ? rsqrt(p) : 0.0;
-		if (!ok && bad == 0) bad = j + 1;
+		// info of an infinite pivot (1 / L_jj = 0, L_jj = inf * 0 = NaN): FP64 looks at
+		// the pivot, FP32 at L_jj, as the FP32 kernel for n > 64 does
+		if ((!ok || (sizeof(T) == 4 && !(p * iv > 0.0))) && bad == 0) bad = j + 1;
 		__syncwarp();
 		for (int i = j + lane; i < n; i += 32)
 			d.at(i, j) = i == j ? (T)(ok ? p * iv : 0.0) : d.at(i, j) * (T)iv;
