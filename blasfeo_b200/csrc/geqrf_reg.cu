@@ -140,7 +140,9 @@ __global__ void __launch_bounds__(NT, MINB)
 				const double sq = seg_sum<SL>(p0 + p1, g, q);
 				const double alpha = seg_sum<SL>(al, g, q);
 				double t = 0.0, sc = 1.0, beta = alpha;
-				if (sq != 0.0) {
+				// (no rows below: no reflector, whatever a NaN or an infinity has left in
+				// the registers of the rows past the last)
+				if (sq != 0.0 && j + 1 < pr) {
 					beta = sqrt(fma(alpha, alpha, sq));
 					if (alpha > 0.0) beta = -beta;
 					t = (beta - alpha) / beta;
