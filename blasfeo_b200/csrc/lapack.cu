@@ -1484,16 +1484,16 @@ inline int pick_geqrf_reg(int batch, int max_m, bool uneven) {
 // not the faster one: its CTA takes the columns right of a panel 16 or 32 at a time
 // with three barriers each, and with more than 128 rows one CTA is all an SM holds.
 // us, register panels / the others: 20 x 1,280 x 1 456 / 149, 8 x 512 x 1 54 / 32,
-// 32 x 256 x 148 108 / 90, 100 x 800 x 148 907 / 802, 160 x 480 x 200 1,571 / 1,237,
+// 32 x 256 x 148 108 / 90, 48 x 768 x 148 365 / 278, 100 x 800 x 148 907 / 802, 160 x 480 x 200 1,571 / 1,237,
 // 300 x 900 x 450 16,427 / 12,036, 2 x 4 x 2,000 13.9 / 10.3; on the other side of
-// the lines 8 x 128 x 1 20 / 23, 32 x 128 x 148 66 / 78, 32 x 512 x 300 240 / 291,
+// the lines 8 x 128 x 1 20 / 23, 40 x 300 x 148 138 / 147, 32 x 128 x 148 66 / 78, 32 x 512 x 300 240 / 291,
 // 160 x 240 x 300 0.88 of the other's time, 256 x 3,072 x 148 0.97.
 inline bool geqrf_wide(int batch, int max_m, int max_n) {
 	const bool few = batch <= bf::num_sms();
 	if (max_m <= 2) return max_n >= 3 && max_n <= 8;
 	if (max_n <= 3) return max_m > 16 && max_m <= 64 && batch > 4 * bf::num_sms();
 	if (max_m > 16 && max_m <= 32 && !few) return batch <= 3 * bf::num_sms() && max_n > 32 * max_m;
-	if (max_m <= 64) return few && max_n > 100 && max_n > (max_m <= 16 ? 22 : (max_m <= 32 ? 6 : 7)) * max_m;
+	if (max_m <= 64) return few && max_n > 100 && max_n > (max_m <= 16 ? 22 : (max_m <= 32 ? 6 : 8)) * max_m;
 	if (max_m <= 128) return max_n > 7 * max_m;
 	if (few) return max_m <= 255 && max_n > 10 * max_m;
 	return max_m <= 256 ? 2 * max_n > 3 * max_m : 5 * max_n > 7 * max_m;
