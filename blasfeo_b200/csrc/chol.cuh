@@ -105,18 +105,6 @@ __device__ __forceinline__ void tri_index(int t, int &ti, int &tj) {
 	tj = t - r * (r + 1) / 2;
 }
 
-// Cholesky pivot through one reciprocal square root: inv = 1/sqrt(c),
-// d = c*inv (= sqrt(c)); non-positive c -> 0, 0.
-__device__ __forceinline__ void chol_pivot_rsqrt(double c, double &d, double &inv) {
-	if (c > 0.0) {
-		inv = rsqrt(c);
-		d = c * inv;
-	} else {
-		d = 0.0;
-		inv = 0.0;
-	}
-}
-
 // Doubles of scratch of the diagonal blocks: the row-major copy Lt (16 x 17,
 // sized for FP64), then what frag::chol16 needs
 constexpr int CHOL_SCR = 16 * 17 + 32;
