@@ -412,6 +412,8 @@ void launch_trs(const SvArgs &a, cudaStream_t s) {
 template <int NU>  // nu <= NU
 __global__ void __launch_bounds__(256)
     k_ric_gains(int batch, int N, int nx, int nu, const double *pL, long long sl, double *pK, long long sk, int cnk) {
+	__shared__ double s_l[NU > 8 ? 16 : 1][NU > 8 ? 16 * 17 : 1];
+	double *ls = s_l[NU > 8 ? threadIdx.x >> 4 : 0];
 	const int i = threadIdx.x & 15;
 	const long long total = (long long)batch * N;
 	const long long step = (long long)gridDim.x * 16;
@@ -427,12 +429,19 @@ __global__ void __launch_bounds__(256)
 		for (int c = 0; c < NU; c++) l[c] = (c < nu && c <= i && i < nu + nx) ? L[pmi(i, c, RV)] : 0.0;
 		const double inv = i < nu ? 1.0 / L[pmi(i, i, RV)] : 0.0;
 		double kc[NU];
+		if constexpr (NU > 8) {
+			// rows of Luu through shared memory: 120 shuffles would take longer
+			__syncwarp();
+#pragma unroll
+			for (int c = 0; c < NU; c++) ls[c * 17 + i] = l[c];
+			__syncwarp();
+		}
 #pragma unroll
 		for (int r = NU - 1; r >= 0; r--) {
 			double c = -l[r];
 #pragma unroll
 			for (int q = r + 1; q < NU; q++) {
-				const double lqr = shh(l[r], q);
+				const double lqr = NU > 8 ? ls[r * 17 + q] : shh(l[r], q);
 				if (q < nu) c = fma(-lqr, kc[q], c);
 			}
 			kc[r] = c * shh(inv, r);
