@@ -160,7 +160,8 @@ __global__ void k_invdiag(SizeArg sz, MatArg<T> A) {
 // broadcast 16-byte loads for 16 FMAs.  The loops over blocks and solved columns
 // are rolled: the form with the whole row in registers (64 columns unrolled,
 // about 8,000 instructions run once per row) was bound by instruction fetch:
-// FP32, m = 60, n = 50 x 6,000 504 us, this kernel 129.  Shared memory:
+// FP32, m = 60, n = 50 x 6,000 504 us, this kernel 119 (ncu: issue slots 50%; a warp
+// waits 2.9 of 9.2 cycles for global memory, 1.8 for shared memory).  Shared memory:
 // A's blocks (8 nb (nb + 1) 16 entries), R columns of 16 nb, the inverse diagonal.
 __host__ __device__ inline size_t trsm_rows_elems(int n, int R) {
 	const int nb = (n + 15) >> 4;

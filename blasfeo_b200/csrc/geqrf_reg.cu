@@ -27,7 +27,11 @@
 // Size classes as in getrf_reg.cu.  1,024 matrices 2n x n, n log-uniform in
 // 4..192: 1.27 -> 0.62 ms; uniform 16 x 8 x 20,000 198 -> 151 us, 64 x 32 x
 // 20,000 3.38 -> 1.35 ms, 128 x 64 x 20,000 13.0 -> 5.3, 384 x 192 x 3,791 19.8 ->
-// 15.7 ms.
+// 15.7 ms.  That uneven batch (512 threads, one CTA per SM; ncu): a warp issues every
+// 14.4 cycles, 5.9 of them at barriers; issue slots 28%, tensor pipe 15%, DRAM 2%.
+// The 128 registers per thread spill (bytes of stores: 284 for up to 384 rows, 560
+// beyond, 152 at 256, 188 with 256 threads).  Matrices much wider than tall go to the
+// blocked kernel (geqrf_wide, lapack.cu).
 #include "common.cuh"
 #include "kernels.cuh"
 

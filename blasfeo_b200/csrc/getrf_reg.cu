@@ -9,7 +9,8 @@
 //      kernel/generic/kernel_dgetrf_pivot_lib4.c:84-165) by three redux per
 //      warp, the warp's candidate row to shared memory, ONE barrier, the
 //      winner among the warps by three more; rows are not moved, the two
-//      positions are exchanged; every thread scales and updates its rows;
+//      positions are exchanged (without pivoting row j goes to shared memory, no
+//      search); every thread scales and updates its rows;
 //   c. the rows go to their positions in D and in shared memory; the positions
 //      are the panel's permutation;
 //   per chunk of at most CH columns right of the panel:
@@ -29,9 +30,12 @@
 // to L2.  Size classes: a variable-size launch starts its CTAs largest first
 // (grid = classes x batch, the CTAs of the other classes leave at once): a
 // 384 x 384 matrix that starts last would otherwise run alone.  1,024 matrices,
-// sizes log-uniform in 4..384: 2.39 -> 0.74 ms; uniform n = 16 x 20,000 0.38 -> 0.11,
+// sizes log-uniform in 4..384: 2.39 -> 0.72 ms; uniform n = 16 x 20,000 0.38 -> 0.11,
 // n = 64 x 20,000 5.39 -> 1.86, n = 256 x 2,013 7.51 -> 3.82, n = 384 x 825
-// 10.7 -> 5.2 ms.
+// 10.7 -> 5.2 ms.  That uneven batch (512 threads, one CTA per SM; ncu): a warp issues
+// every 11.6 cycles, 4.0 of them at barriers; issue slots 34%, tensor pipe 9%, DRAM
+// 6%.  The 128 registers per thread spill (224 bytes of stores, 172 without
+// pivoting).
 #include "common.cuh"
 #include "kernels.cuh"
 

@@ -573,8 +573,10 @@ constexpr int POSV_GLOBAL_MINB = 4;
 // go to loads in flight: two fragment rows by four steps of 8 columns in the
 // panel update at 4 CTAs per SM (5,000 systems, n ~ U{4..256}: 1,102 us; one
 // fragment row 1,155, and at 5 / 6 CTAs with spills 1,332 / 1,370; eight steps
-// 1,197).  With the substitutions apart, L read step by step inside them, and
-// the other warps idle during the diagonal blocks: 1,635.
+// 1,197; all before the systems from n = 65 on came here and the diagonal factor
+// moved into the panel: 1,063 now).  The 128 registers spill (320 bytes of stores).
+// With the substitutions apart, L read step by step inside them, and the other warps
+// idle during the diagonal blocks: 1,635.
 __global__ void __launch_bounds__(POSV_GLOBAL_NT, POSV_GLOBAL_MINB)
     k_posv_global(int cls, int max_n, PosvWs ws, const int *__restrict__ nvec, const DevDesc<double> *__restrict__ sA,
                   const DevVec<double> *__restrict__ sb, const DevVec<double> *__restrict__ sx, double *slots,

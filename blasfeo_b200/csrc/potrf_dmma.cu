@@ -23,11 +23,15 @@
 // take afterwards), so the sum is never written: FP32 n = 50, k = 37 x 6,000 as
 // two launches 125 + 127 us, this kernel 109.
 //
-// Bound: the pivot chain (two pivots per 220 cycles) with the warps that the
-// registers allow (8 per SM at n = 64), then the FP64 tensor pipe (384 steps of
-// 15 cycles per SM sub-partition at n = 64).  8,000 matrices of n = 64: pivots,
-// rows and columns broadcast by shuffles 171 us, this form 155 us (n = 48:
-// 21,000 matrices 526 -> 309 us, n = 32: 40,000 198 -> 150 us).
+// Bound: latency with the two warps per SM sub-partition that the registers allow
+// (n = 64): a matrix is about 6,000 instructions, and a warp issues one every 7.6
+// cycles (ncu: 2.8 of them waiting for an earlier result, 1.1 for the FP64 pipe, 0.7
+// for shared memory, 0.6 for global memory, 0.5 for instructions; issue slots 26%
+// used, the pipe 38%), 45,000 cycles a matrix.  The pivots themselves (two per 220
+// cycles, 7,000 a matrix) and the tensor steps (384 of 15 cycles) are the smaller
+// part.  8,000 matrices of n = 64: pivots, rows and columns broadcast by shuffles 171
+// us, this form 156 (n = 48: 21,000 matrices 526 -> 309 us, n = 32: 40,000 198 -> 150).
+// With the product the fragments of n = 41..48 spill (208 bytes of stores in FP32).
 #include "chol_frag.cuh"
 #include "kernels.cuh"
 

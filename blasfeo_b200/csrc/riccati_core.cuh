@@ -23,15 +23,18 @@
 //     gets the first one's update in two steps.  No shuffles: a 64-bit shuffle
 //     occupies the SM's shuffle unit for about 8 cycles, and the quad and
 //     half-warp forms of the factorization need 272 of them per warp, which
-//     bounded them (4,096 problems, N = 30, 12 + 4, interleaved: quads 0.281
-//     ms, 8 lanes 0.271, 16 lanes 0.275; this kernel 0.261).
+//     bounded them (4,096 problems, N = 30, 12 + 4, interleaved: quads 0.277
+//     ms, 8 lanes 0.271, 16 lanes 0.275; this kernel 0.268, back to back 0.232
+//     against 0.88 for a warp with FMAs and shuffles).
 // The next stage's inputs arrive by cp.async under the factorization.
 //
-// What bounds it: the chain of 16 pivots per stage (shared memory, reciprocal
-// square root, scale, tensor core step: about 130 cycles each) with 28 problems
-// per SM to hide it, then instruction issue (900 per problem and stage) and the
-// FP64 tensor pipe (40 steps of 15 cycles); the bytes (BAbt, lower RSQ in;
-// lower L out: 0.073 ms there) are the floor.
+// What bounds it: latency with 7 warps per SM sub-partition, each a stage of 31
+// after another.  Back to back issue slots are 60% and the FP64 pipe 53% used (ncu;
+// a warp issues every 10.2 cycles: 2.9 waiting for an earlier result, 2.5 for the pipe,
+// 1.3 for shared memory); interleaved 45% and 45%, with 2.8 cycles for shared memory
+// and 1.4 for its queue: one 8-byte copy per element and lane instead of 16-byte
+// ones, and CTA barriers in the place of warp barriers.  The bytes (BAbt, lower RSQ
+// in; lower L out: 0.073 ms there) are the floor.
 #pragma once
 
 #include "chol_frag.cuh"

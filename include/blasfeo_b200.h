@@ -426,8 +426,8 @@ int blasfeo_dgeqrf_vbatch(int batch, const int *m, const int *n, int max_m, int 
  *   memory, 5 one warp per instance on the FP64 tensor cores (max_m <= 64;
  *   larger batches take the heuristic);
  * op 2 getrf_rp: 0..2 blocked with the panel in registers, 128 (fewer for up to
- *   64 rows), 256 and 512 threads per matrix (more than 512 rows: blocked in
- *   global memory), 3..5 shared memory with 128/256/512 threads;
+ *   64 rows and 128 columns), 256 and 512 threads per matrix (more than 512 rows:
+ *   blocked in global memory), 3..5 shared memory with 128/256/512 threads;
  * op 3 geqrf: 0..2 blocked with the panel in registers, 128 (64 for up to 32
  *   rows), 256 and 512 threads per matrix (more threads where the rows need
  *   them; more than 512 rows: blocked in global memory), 3..5 shared memory with
