@@ -1488,7 +1488,9 @@ inline int pick_geqrf_reg(int batch, int max_m, bool uneven) {
 // 32 x 256 x 148 108 / 90, 48 x 768 x 148 365 / 278, 100 x 800 x 148 907 / 802, 160 x 480 x 200 1,571 / 1,237,
 // 300 x 900 x 450 16,427 / 12,036, 2 x 4 x 2,000 13.9 / 10.3; on the other side of
 // the lines 8 x 128 x 1 20 / 23, 40 x 300 x 148 138 / 147, 32 x 128 x 148 66 / 78, 32 x 512 x 300 240 / 291,
-// 160 x 240 x 300 0.88 of the other's time, 256 x 3,072 x 148 0.97.
+// 160 x 240 x 300 0.88 of the other's time, 256 x 3,072 x 148 0.97.  An uneven batch
+// is judged by its largest rows and columns, which need not belong to one matrix: 4
+// log-uniform ones of up to 16 x 500, 40 x 400, 100 x 800 30 / 40, 73 / 97, 244 / 313.
 inline bool geqrf_wide(int batch, int max_m, int max_n) {
 	const bool few = batch <= bf::num_sms();
 	if (max_m <= 2) return max_n >= 3 && max_n <= 8;
